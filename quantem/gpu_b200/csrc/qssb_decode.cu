@@ -19,9 +19,12 @@
 // bit-unshuffles the block with 8x8 bit transposes straight into the u16
 // frame (16-byte stores). A malformed chunk sets status[c] (the block is
 // zero-filled); nothing traps.
-// Encode: the same transposes forward, a greedy LZ4 compressor per block
-// (lane 0, a 4096-entry hash table in shared memory) into fixed-stride
-// slots, then a pack kernel that lays out the chunks at caller offsets.
+// Encode: a warp per block makes the same transposes forward and the greedy
+// LZ4 of a serial search (32 positions a step, a 4096-entry hash table in
+// shared memory) into fixed-stride slots, then a pack kernel lays out the
+// chunks at caller offsets.
+#include <limits.h>
+
 #include "qssb_internal.h"
 
 namespace qssb {
@@ -234,90 +237,150 @@ __global__ void __launch_bounds__(32 * kDecWarps) k_decode_bslz4_u16(
 // Scratch layout: per (chunk, block) a slot of kEncSlot bytes holding the
 // big-endian compressed size followed by the LZ4 block.
 constexpr int kEncSlot = (4 + kLz4Bound + 15) & ~15;
+constexpr int kEncWarps = 4;
+// planes | hash table; the warps of a CTA share nothing
+constexpr int kEncWarpBytes = kBlockBytes + 2 * kEncHash;
 
-__device__ __forceinline__ uint32_t rd32(const uint8_t* p) {
-    return (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
+// Four bytes at any byte position of a 4-aligned shared buffer. The second
+// word of an aligned position is read (it may be the first word of the hash
+// table) and shifted out.
+__device__ __forceinline__ uint32_t rd32(const uint8_t* base, int pos) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(base) + (pos >> 2);
+    return __funnelshift_r(w[0], w[1], 8 * (pos & 3));
 }
 
-__global__ void __launch_bounds__(32 * kDecWarps) k_encode_bslz4_u16(
-    const uint16_t* __restrict__ frames, int n_chunks, long long chunk_bytes,
+// LZ4 length extension: x / 255 bytes of 255, then the rest. Returns the bytes written.
+__device__ __forceinline__ int put_length(uint8_t* o, int x, int lane) {
+    const int q = x / 255;
+    for (int k = lane; k <= q; k += 32) o[k] = (uint8_t)(k < q ? 255 : x - 255 * q);
+    return q + 1;
+}
+
+// The greedy LZ4 of one block in shared memory by a whole warp, with the
+// bytes of the serial search: every position from ip on looks up the last
+// position of its 12-bit hash and enters itself, until the first whose four
+// bytes match. The 32 lanes take positions ip .. ip + 31 at once: a lane's
+// candidate is the nearest lower lane of the same hash (__match_any_sync) or
+// the table's entry, the first hit is the lowest set bit of a ballot, and
+// only lanes up to it enter the table (the highest of each hash). Matches are
+// extended 128 bytes a step, literals copied 32 bytes a step.
+__device__ int lz4_encode_block_warp(const uint8_t* planes, int n, uint16_t* table, uint8_t* o,
+                                     int lane) {
+    int op = 0, anchor = 0, ip = 0;
+    const int last = n - 12;  // no match starts in the last 12 bytes
+    while (ip < last) {
+        const int pos = ip + lane;
+        const bool on = pos < last;
+        const uint32_t v = rd32(planes, on ? pos : ip);
+        const uint32_t h = on ? (v * 2654435761u) >> 20 : kEncHash;  // idle lanes: a hash of their own
+        const unsigned same = __match_any_sync(0xffffffffu, h);
+        const unsigned below = same & ((1u << lane) - 1u);
+        int cand = 0xffff;
+        if (on) cand = below ? ip + 31 - __clz(below) : (int)table[h];
+        const bool hit = cand != 0xffff && rd32(planes, cand) == v;
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        const int first = hits ? __ffs(hits) - 1 : 31;
+        // a lane at or before the first hit enters its position unless a later
+        // such lane has its hash (lanes beyond `last` have none)
+        if (on && lane <= first && (same & (0xffffffffu >> (31 - first))) >> lane == 1u)
+            table[h] = (uint16_t)pos;
+        __syncwarp();
+        if (!hits) {
+            ip += 32;
+            continue;
+        }
+        ip += first;
+        cand = __shfl_sync(0xffffffffu, cand, first);
+        int m = 4;
+        const int room = n - 5 - ip;  // the last 5 bytes stay literal
+        for (;;) {
+            const int at = m + 4 * lane;
+            int eq = 0;  // equal bytes of this lane's four
+            if (at < room) {
+                const uint32_t x = rd32(planes, ip + at) ^ rd32(planes, cand + at);
+                eq = min(x ? (__ffs(x) - 1) >> 3 : 4, room - at);
+            }
+            const unsigned stop = __ballot_sync(0xffffffffu, eq < 4);
+            if (stop) {
+                const int l = __ffs(stop) - 1;
+                m += 4 * l + __shfl_sync(0xffffffffu, eq, l);
+                break;
+            }
+            m += 128;
+        }
+        const int lit = ip - anchor;
+        if (lane == 0) o[op] = (uint8_t)((min(lit, 15) << 4) | min(m - 4, 15));
+        ++op;
+        if (lit >= 15) op += put_length(o + op, lit - 15, lane);
+        for (int k = lane; k < lit; k += 32) o[op + k] = planes[anchor + k];
+        op += lit;
+        const int off = ip - cand;
+        if (lane < 2) o[op + lane] = (uint8_t)(off >> (8 * lane));
+        op += 2;
+        if (m - 4 >= 15) op += put_length(o + op, m - 4 - 15, lane);
+        ip += m;
+        anchor = ip;
+    }
+    const int lit = n - anchor;
+    if (lane == 0) o[op] = (uint8_t)(min(lit, 15) << 4);
+    ++op;
+    if (lit >= 15) op += put_length(o + op, lit - 15, lane);
+    for (int k = lane; k < lit; k += 32) o[op + k] = planes[anchor + k];
+    return op + lit;
+}
+
+// One warp per (chunk, block), blocks of one chunk in consecutive warps.
+// Bound by the latency of a window's shared-memory chain (hash, table,
+// candidate bytes, ballots) times the windows of a block, so the launch is as
+// many warps as the 16 KB of planes and table of each allow. 4096 frames of
+// 128 x 128 counts: the whole call 0.73 ms against 4.00 ms with one lane
+// searching byte by byte and copying (the same bytes).
+__global__ void __launch_bounds__(32 * kEncWarps) k_encode_bslz4_u16(
+    const uint16_t* __restrict__ frames, long long n_slots, int n_blocks, long long chunk_bytes,
     uint8_t* __restrict__ scratch) {
     extern __shared__ uint4 enc_smem4[];
-    uint8_t* base = reinterpret_cast<uint8_t*>(enc_smem4);
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = tid >> 5;
-    const int c = blockIdx.x;
+    const int lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const long long item = (long long)blockIdx.x * kEncWarps + warp;
+    if (item >= n_slots) return;
+    const long long c = item / n_blocks;
+    const int i = (int)(item - c * n_blocks);
     const long long n_elem = chunk_bytes / 2;
     const long long n8 = n_elem & ~7LL;
-    const int n_blocks = (int)((n8 + kBlockElems - 1) / kBlockElems);
-    uint8_t* planes = base + (size_t)warp * (kBlockBytes + 2 * kEncHash);
+    uint8_t* planes = reinterpret_cast<uint8_t*>(enc_smem4) + (size_t)warp * kEncWarpBytes;
     uint16_t* table = reinterpret_cast<uint16_t*>(planes + kBlockBytes);
-    const uint16_t* frame = frames + (size_t)c * n_elem;
-    for (int i = warp; i < n_blocks; i += kDecWarps) {
-        const long long e0 = (long long)i * kBlockElems;
-        const int cnt = (int)min((long long)kBlockElems, n8 - e0);
-        const int P = cnt / 8;
-        for (int p = lane; p < P; p += 32) {  // forward bit shuffle
-            uint64_t lo = 0, hi = 0;
+    const long long e0 = (long long)i * kBlockElems;
+    const uint16_t* src = frames + (size_t)c * n_elem + e0;
+    const int cnt = (int)min((long long)kBlockElems, n8 - e0);
+    const int P = cnt / 8;
+    const bool vec = ((uintptr_t)src & 15u) == 0;
+    for (int p = lane; p < P; p += 32) {  // forward bit shuffle
+        uint32_t w[4];
+        if (vec) {
+            const uint4 q = __ldcs(reinterpret_cast<const uint4*>(src) + p);
+            w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
+        } else {
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint16_t v = frame[e0 + 8 * p + j];
-                lo |= (uint64_t)(v & 0xff) << (8 * j);
-                hi |= (uint64_t)(v >> 8) << (8 * j);
-            }
-            lo = transpose8(lo);
-            hi = transpose8(hi);
+            for (int j = 0; j < 4; ++j)
+                w[j] = (uint32_t)src[8 * p + 2 * j] | ((uint32_t)src[8 * p + 2 * j + 1] << 16);
+        }
+        // low and high bytes of the 8 elements
+        const uint64_t lo = transpose8((uint64_t)__byte_perm(w[0], w[1], 0x6420) |
+                                       ((uint64_t)__byte_perm(w[2], w[3], 0x6420) << 32));
+        const uint64_t hi = transpose8((uint64_t)__byte_perm(w[0], w[1], 0x7531) |
+                                       ((uint64_t)__byte_perm(w[2], w[3], 0x7531) << 32));
 #pragma unroll
-            for (int b = 0; b < 8; ++b) {
-                planes[b * P + p] = (uint8_t)(lo >> (8 * b));
-                planes[(8 + b) * P + p] = (uint8_t)(hi >> (8 * b));
-            }
+        for (int b = 0; b < 8; ++b) {
+            planes[b * P + p] = (uint8_t)(lo >> (8 * b));
+            planes[(8 + b) * P + p] = (uint8_t)(hi >> (8 * b));
         }
-        for (int h = lane; h < kEncHash; h += 32) table[h] = 0xffff;
-        __syncwarp();
-        if (lane == 0) {  // greedy LZ4 (last 5 bytes literal, no match in the last 12)
-            const int n = 2 * cnt;
-            uint8_t* slot = scratch + ((size_t)c * n_blocks + i) * kEncSlot;
-            uint8_t* o = slot + 4;
-            int op = 0, anchor = 0, ip = 0;
-            auto put_len = [&](int x) {
-                while (x >= 255) { o[op++] = 255; x -= 255; }
-                o[op++] = (uint8_t)x;
-            };
-            while (ip < n - 12) {
-                const uint32_t v = rd32(planes + ip);
-                const uint32_t h = (v * 2654435761u) >> 20;
-                const int cand = table[h];
-                table[h] = (uint16_t)ip;
-                if (cand != 0xffff && rd32(planes + cand) == v) {
-                    int m = 4;
-                    while (ip + m < n - 5 && planes[cand + m] == planes[ip + m]) ++m;
-                    const int lit = ip - anchor;
-                    o[op++] = (uint8_t)((min(lit, 15) << 4) | min(m - 4, 15));
-                    if (lit >= 15) put_len(lit - 15);
-                    for (int k = 0; k < lit; ++k) o[op++] = planes[anchor + k];
-                    const int off = ip - cand;
-                    o[op++] = (uint8_t)(off & 0xff);
-                    o[op++] = (uint8_t)(off >> 8);
-                    if (m - 4 >= 15) put_len(m - 4 - 15);
-                    ip += m;
-                    anchor = ip;
-                } else {
-                    ++ip;
-                }
-            }
-            const int lit = n - anchor;
-            o[op++] = (uint8_t)(min(lit, 15) << 4);
-            if (lit >= 15) put_len(lit - 15);
-            for (int k = 0; k < lit; ++k) o[op++] = planes[anchor + k];
-            slot[0] = (uint8_t)(op >> 24);
-            slot[1] = (uint8_t)(op >> 16);
-            slot[2] = (uint8_t)(op >> 8);
-            slot[3] = (uint8_t)op;
-        }
-        __syncwarp();
     }
+    uint4* t4 = reinterpret_cast<uint4*>(table);
+    for (int h = lane; h < kEncHash / 8; h += 32) t4[h] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    __syncwarp();
+    uint8_t* slot = scratch + (size_t)item * kEncSlot;
+    const int op = lz4_encode_block_warp(planes, 2 * cnt, table, slot + 4, lane);
+    if (lane < 4) slot[lane] = (uint8_t)(op >> (24 - 8 * lane));
 }
 
 // sizes[c] = bytes of chunk c: header, the blocks with their size words, raw leftovers.
@@ -333,34 +396,62 @@ __global__ void k_bslz4_chunk_sizes(const uint8_t* __restrict__ scratch, int n_c
     sizes[c] = total;
 }
 
-__global__ void __launch_bounds__(256) k_bslz4_pack(const uint8_t* __restrict__ scratch,
-                                                    const uint16_t* __restrict__ frames,
-                                                    int n_chunks, long long chunk_bytes,
-                                                    const long long* __restrict__ offsets,
-                                                    uint8_t* __restrict__ packed) {
-    const int c = blockIdx.x;
-    const int tid = threadIdx.x;
+// One warp per (chunk, block): the block's slot to its place in the chunk
+// (the sizes of the chunk's earlier blocks summed by the lanes), 16 bytes a
+// lane on the destination's alignment, the source words funnel-shifted. The
+// first block's warp writes the chunk header, the last one's the raw leftovers.
+constexpr int kPackWarps = 8;
+__global__ void __launch_bounds__(32 * kPackWarps) k_bslz4_pack(
+    const uint8_t* __restrict__ scratch, const uint16_t* __restrict__ frames, long long n_items,
+    int n_blocks, long long chunk_bytes, const long long* __restrict__ offsets,
+    uint8_t* __restrict__ packed) {
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * kPackWarps + (threadIdx.x >> 5);
+    if (item >= n_items) return;
+    const int per = max(n_blocks, 1);  // a chunk of fewer than 8 elements has no block
+    const long long c = item / per;
+    const int i = (int)(item - c * per);
     const long long n_elem = chunk_bytes / 2;
     const long long n8 = n_elem & ~7LL;
-    const int n_blocks = (int)((n8 + kBlockElems - 1) / kBlockElems);
     uint8_t* dst = packed + offsets[c];
-    if (tid < 12) {
-        dst[tid] = tid < 8 ? (uint8_t)((unsigned long long)chunk_bytes >> (8 * (7 - tid)))
-                           : (uint8_t)((uint32_t)kBlockBytes >> (8 * (11 - tid)));
+    if (i == 0 && lane < 12) {
+        dst[lane] = lane < 8 ? (uint8_t)((unsigned long long)chunk_bytes >> (8 * (7 - lane)))
+                             : (uint8_t)((uint32_t)kBlockBytes >> (8 * (11 - lane)));
     }
-    long long pos = 12;
-    for (int i = 0; i < n_blocks; ++i) {
-        const uint8_t* slot = scratch + ((size_t)c * n_blocks + i) * kEncSlot;
-        const int len = 4 + (int)be32(slot);
-        for (int j = tid; j < len; j += 256) dst[pos + j] = slot[j];
-        pos += len;
+    const uint8_t* first = scratch + (size_t)c * n_blocks * kEncSlot;
+    int before = 0;
+    for (int j = lane; j < i; j += 32) before += 4 + (int)be32(first + (size_t)j * kEncSlot);
+    dst += 12 + __reduce_add_sync(0xffffffffu, before);
+    const uint8_t* slot = first + (size_t)i * kEncSlot;
+    const int len = n_blocks ? 4 + (int)be32(slot) : 0;
+    const int head = min(len, (int)((16u - ((uintptr_t)dst & 15u)) & 15u));
+    if (lane < head) dst[lane] = slot[lane];
+    const int n_vec = (len - head) >> 4;
+    const int shift = 8 * (head & 3);
+    const uint32_t* words = reinterpret_cast<const uint32_t*>(slot) + (head >> 2);
+    uint4* out = reinterpret_cast<uint4*>(dst + head);
+    for (int t = lane; t < n_vec; t += 32) {
+        const uint32_t* w = words + 4 * t;
+        const uint32_t w4 = shift ? w[4] : 0u;  // within the slot: it holds needed bytes
+        const uint32_t w1 = w[1], w2 = w[2], w3 = w[3];
+        out[t] = make_uint4(__funnelshift_r(w[0], w1, shift), __funnelshift_r(w1, w2, shift),
+                            __funnelshift_r(w2, w3, shift), __funnelshift_r(w3, w4, shift));
     }
+    const int done = head + 16 * n_vec;
+    if (done + lane < len) dst[done + lane] = slot[done + lane];
+    if (i + 1 < n_blocks) return;
     const uint16_t* frame = frames + (size_t)c * n_elem;
-    for (long long j = n8 + tid; j < n_elem; j += 256) {
+    for (long long j = n8 + lane; j < n_elem; j += 32) {
         const uint16_t v = frame[j];
-        dst[pos + 2 * (j - n8)] = (uint8_t)(v & 0xff);
-        dst[pos + 2 * (j - n8) + 1] = (uint8_t)(v >> 8);
+        dst[len + 2 * (j - n8)] = (uint8_t)(v & 0xff);
+        dst[len + 2 * (j - n8) + 1] = (uint8_t)(v >> 8);
     }
+}
+
+// The shuffled blocks of one chunk.
+static int chunk_blocks(long long chunk_bytes) {
+    const long long n8 = (chunk_bytes / 2) & ~7LL;
+    return (int)((n8 + kBlockElems - 1) / kBlockElems);
 }
 
 static int check_chunk_bytes(long long chunk_bytes, const char* who) {
@@ -399,9 +490,7 @@ extern "C" int qssb_encode_bslz4_scratch_bytes(int32_t n_chunks, int64_t chunk_b
     int rc = check_chunk_bytes(chunk_bytes, "qssb_encode_bslz4_scratch_bytes: chunk_bytes must be "
                                             "even, at most 4 MB");
     if (rc) return rc;
-    const long long n8 = (chunk_bytes / 2) & ~7LL;
-    const long long n_blocks = (n8 + kBlockElems - 1) / kBlockElems;
-    *bytes = (size_t)n_chunks * (size_t)n_blocks * kEncSlot;
+    *bytes = (size_t)n_chunks * (size_t)chunk_blocks(chunk_bytes) * kEncSlot;
     return QSSB_OK;
 }
 
@@ -413,11 +502,16 @@ extern "C" int qssb_encode_bslz4_u16(const uint16_t* frames, int32_t n_chunks, i
                                             "at most 4 MB");
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const size_t smem = (size_t)kDecWarps * (kBlockBytes + 2 * kEncHash);
-    CUDA_TRY(cudaFuncSetAttribute(k_encode_bslz4_u16, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    { k_encode_bslz4_u16<<<n_chunks, 32 * kDecWarps, smem, s>>>(frames, n_chunks, chunk_bytes, scratch); note_launch(); }
-    CUDA_TRY(cudaGetLastError());
+    const int n_blocks = chunk_blocks(chunk_bytes);
+    const long long n_slots = (long long)n_chunks * n_blocks;
+    if (n_slots > 0) {
+        const int smem = kEncWarps * kEncWarpBytes;
+        const long long grid = (n_slots + kEncWarps - 1) / kEncWarps;
+        if (grid > INT_MAX) return set_error(QSSB_ERR_INVALID, "qssb_encode_bslz4_u16: too many blocks");
+        CUDA_TRY(cudaFuncSetAttribute(k_encode_bslz4_u16, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        { k_encode_bslz4_u16<<<(unsigned)grid, 32 * kEncWarps, smem, s>>>(frames, n_slots, n_blocks, chunk_bytes, scratch); note_launch(); }
+        CUDA_TRY(cudaGetLastError());
+    }
     { k_bslz4_chunk_sizes<<<(n_chunks + 255) / 256, 256, 0, s>>>(
         scratch, n_chunks, chunk_bytes, reinterpret_cast<long long*>(chunk_sizes)); note_launch(); }
     CUDA_TRY(cudaGetLastError());
@@ -431,9 +525,13 @@ extern "C" int qssb_pack_bslz4(const uint8_t* scratch, const uint16_t* frames, i
         return set_error(QSSB_ERR_INVALID, "qssb_pack_bslz4: null pointer or empty input");
     int rc = check_chunk_bytes(chunk_bytes, "qssb_pack_bslz4: chunk_bytes must be even, at most 4 MB");
     if (rc) return rc;
-    { k_bslz4_pack<<<n_chunks, 256, 0, (cudaStream_t)stream>>>(
-        scratch, frames, n_chunks, chunk_bytes, reinterpret_cast<const long long*>(chunk_offsets),
-        packed); note_launch(); }
+    const int n_blocks = chunk_blocks(chunk_bytes);
+    const long long n_items = (long long)n_chunks * (n_blocks > 0 ? n_blocks : 1);
+    const long long grid = (n_items + kPackWarps - 1) / kPackWarps;
+    if (grid > INT_MAX) return set_error(QSSB_ERR_INVALID, "qssb_pack_bslz4: too many blocks");
+    { k_bslz4_pack<<<(unsigned)grid, 32 * kPackWarps, 0, (cudaStream_t)stream>>>(
+        scratch, frames, n_items, n_blocks, chunk_bytes,
+        reinterpret_cast<const long long*>(chunk_offsets), packed); note_launch(); }
     CUDA_TRY(cudaGetLastError());
     return QSSB_OK;
 }

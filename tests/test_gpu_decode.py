@@ -125,3 +125,66 @@ def test_ssb_from_chunks_matches_from_array():
     b = SSB.from_chunks(packed.cpu().pin_memory(), chunk_offsets=offsets.cpu(), frame_shape=(64, 64),
                         scan_shape=(32, 32), **kw).reconstruct(ab)
     assert torch.equal(a.object_wave, want) and torch.equal(b.object_wave, want)
+
+
+def _serial_lz4(src: bytes) -> bytes:
+    """The encoder's search one position at a time: the last position of each
+    12-bit hash, entered at every position looked at."""
+    n, out, anchor, ip, table = len(src), bytearray(), 0, 0, {}
+
+    def length(x):
+        return b"\xff" * (x // 255) + bytes([x % 255])
+
+    def literals(end, extra):
+        lit = end - anchor
+        out.append(min(lit, 15) << 4 | extra)
+        if lit >= 15:
+            out.extend(length(lit - 15))
+        out.extend(src[anchor:end])
+
+    while ip < n - 12:
+        h = (int.from_bytes(src[ip:ip + 4], "little") * 2654435761 & 0xFFFFFFFF) >> 20
+        cand, table[h] = table.get(h), ip
+        if cand is None or src[cand:cand + 4] != src[ip:ip + 4]:
+            ip += 1
+            continue
+        m = 4
+        while ip + m < n - 5 and src[cand + m] == src[ip + m]:
+            m += 1
+        literals(ip, min(m - 4, 15))
+        out.extend((ip - cand).to_bytes(2, "little"))
+        if m - 4 >= 15:
+            out.extend(length(m - 19))
+        ip += m
+        anchor = ip
+    literals(n, 0)
+    return bytes(out)
+
+
+@pytest.mark.parametrize("shape", [(1, 8), (1, 23), (64, 64), (64, 65), (67, 62), (128, 96)])
+@pytest.mark.parametrize("kind", ["zeros", "dense", "counts", "period", "collide"])
+def test_encoder_writes_the_serial_search_bytes(shape, kind):
+    """Blocks of 8 elements up to several blocks with a remainder; runs longer
+    than a step, no match at all, matches of every distance, one hash shared by
+    lanes of a step."""
+    rng = np.random.default_rng(shape[0] * 131 + shape[1])
+    n = shape[0] * shape[1]
+    frames = np.zeros((3, *shape), np.uint16)
+    if kind == "dense":
+        frames = rng.integers(0, 65536, frames.shape, dtype=np.uint16)
+    elif kind == "counts":
+        frames = _frames(3, shape, seed=n)
+    elif kind == "period":
+        frames[:] = np.resize(np.repeat(rng.integers(0, 65536, 7, dtype=np.uint16), 11), frames.shape)
+    elif kind == "collide":
+        frames[:] = np.where(rng.random(frames.shape) < 0.03, 1, 0)
+    packed, offsets = encode_bslz4(torch.as_tensor(frames, device=DEV))
+    want = []
+    for f in frames.reshape(3, n):
+        chunk = struct.pack(">QI", 2 * n, 8192)
+        for e0 in range(0, n // 8 * 8, 4096):
+            comp = _serial_lz4(bo.bitshuffle(f[e0:min(e0 + 4096, n // 8 * 8)]))
+            chunk += struct.pack(">I", len(comp)) + comp
+        want.append(chunk + f[n // 8 * 8:].tobytes())
+    assert offsets.cpu().tolist() == [0, len(want[0]), len(want[0]) + len(want[1])]
+    assert packed.cpu().numpy().tobytes() == b"".join(want)
