@@ -3,15 +3,15 @@
 // Restates the drift-corrected complex mean of the reference's temporal
 // helpers (ssb/temporal.py:77-257 of bobleesj/quantem.gpu):
 //   fourier_shift: O'_t = ifft2(fft2(O_t) exp(-2 pi i (f_r s_r + f_c s_c))),
-//     f = fftfreq(n, 1) (temporal.py:77-107), as three passes over the stack:
-//     row FFTs; per column strip: FFT along the rows, the ramp, inverse FFT;
-//     inverse row FFTs with the 1 / (R C) scale;
+//     f = fftfreq(n, 1) (temporal.py:77-107), as two passes over the stack:
+//     the rows' transform, ramp in f_c and inverse transform, then the
+//     columns' with the ramp in f_r;
 //   join: with phase reference "first", frames t > 0 are multiplied by
 //     exp(-i angle(sum_p O'_t conj O'_0)) (temporal.py:154-160; the overlap
 //     summed in FP64 in a fixed order), then joined = sum_t w_t O'_t
 //     (temporal.py:234).
-// Line transforms: the warp FFT at 256..1024 points, the shared-memory
-// Stockham transform at 64 and 128.
+// Line transforms: the warp FFT at 256..1024 points, groups of 8 lanes at
+// 128, the shared-memory Stockham transform at 64.
 #include <math.h>
 
 #include "qssb_internal.h"
@@ -44,190 +44,276 @@ __device__ __forceinline__ void line_transform(float2* line, const float2* tw, i
     }
 }
 
-// One warp per row of every frame: out = (scale) * FFT_DIR(row of in).
-template <int C, int DIR>
-__global__ void __launch_bounds__(32 * kTmpWarps) k_tmp_rows(const float2* __restrict__ in,
-                                                             float2* __restrict__ out, int rows,
-                                                             float scale) {
-    constexpr int L = tmp_line<C>();
-    extern __shared__ float2 tmp_rows_smem[];
-    float2* tw = tmp_rows_smem;
-    float2* lines = tw + C;
+// exp(-2 pi i f_k shift) / N, f = fftfreq(N, 1), for a line's N frequencies:
+// the phase is formed in FP64 and reduced before the float32 sincos (the
+// scale is a power of two). Computed once per CTA, whose lines share it.
+template <int N>
+__device__ __forceinline__ void fill_ramp(float2* ramp, float shift, int tid, int threads) {
+    for (int k = tid; k < N; k += threads) {
+        double ph = -((double)(k < N / 2 ? k : k - N) * (1.0 / N)) * (double)shift;  // in turns
+        ph -= rint(ph);
+        float s, co;
+        sincospif((float)(2.0 * ph), &s, &co);
+        ramp[k] = make_float2(co * (1.0f / N), s * (1.0f / N));
+    }
+}
+
+// A line of 128 held by a group of 8 lanes as v[n1] = x[s + 8 n1], shifted:
+// transform, ramp, inverse transform. Both transforms leave X[s + 8 h + 16 k]
+// in v[8 h + k], which is the lane's own value n1 = h + 2 k, so the order
+// between and after them is a renaming of registers.
+__device__ __forceinline__ void shift_line128(float2 (&v)[16], float2* T, int s, const float2* tw,
+                                              const float2* ramp) {
+    fft128_g8<-1>(v, T, s, tw);
+    float2 u[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+        const int n1 = (t >> 3) + 2 * (t & 7);
+        u[n1] = cmul(v[t], ramp[s + 8 * n1]);
+    }
+    fft128_g8<+1>(u, T, s, tw);
+#pragma unroll
+    for (int t = 0; t < 16; ++t) v[(t >> 3) + 2 * (t & 7)] = u[t];
+}
+
+// The shift ramp is separable, so each direction is shifted in one pass
+// (transform, ramp, inverse transform of a line on chip) and the stack goes
+// through memory twice. Row transforms, columns with the 2D ramp and inverse
+// row transforms took 23 + 49 + 23 us at 256 frames of 128^2 (all kernels of
+// the join 185 us); the join of them with both passes and its reductions here
+// takes 92 us in all, against 227.
+// Rows: 128 points as four lines per warp in registers; other sizes a warp
+// per line in shared memory.
+template <int C>
+__host__ __device__ constexpr int shift_lines() { return C == 128 ? 4 * kTmpWarps : kTmpWarps; }
+
+template <int C>
+__host__ __device__ constexpr size_t shift_smem() {
+    return sizeof(float2) * (2 * C + (C == 128 ? (size_t)4 * kTmpWarps * kG8Scratch
+                                               : (size_t)kTmpWarps * (tmp_line<C>() | 1)));
+}
+
+template <int C>
+__global__ void __launch_bounds__(32 * kTmpWarps) k_shift_rows(const float2* __restrict__ in,
+                                                               float2* __restrict__ out, int rows,
+                                                               const float* __restrict__ shifts) {
+    extern __shared__ float2 tmp_smem[];
+    float2* tw = tmp_smem;
+    float2* ramp = tw + C;
+    float2* scratch = ramp + C;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
     fill_twiddles<C>(tw, tid, 32 * kTmpWarps);
+    fill_ramp<C>(ramp, __ldg(shifts + 2 * blockIdx.y + 1), tid, 32 * kTmpWarps);
     __syncthreads();
-    const int r = blockIdx.x * kTmpWarps + warp;
-    if (r >= rows) return;
-    const size_t base = ((size_t)blockIdx.y * rows + r) * C;
-    float2* line = lines + warp * L;
-    for (int i = lane; i < C; i += 32) line[i] = in[base + i];
-    __syncwarp();
-    line_transform<C, DIR>(line, tw, lane);
-    for (int i = lane; i < C; i += 32) {
-        const float2 v = line[i];
-        out[base + i] = make_float2(v.x * scale, v.y * scale);
+    if constexpr (C == 128) {
+        const int group = tid >> 3;
+        const int s = lane & 7;
+        const int r = blockIdx.x * shift_lines<C>() + group;
+        const bool on = r < rows;  // whole warps call the transform
+        const size_t base = ((size_t)blockIdx.y * rows + (on ? r : 0)) * C;
+        float2 v[16];
+#pragma unroll
+        for (int n1 = 0; n1 < 16; ++n1) v[n1] = in[base + s + 8 * n1];
+        shift_line128(v, scratch + group * kG8Scratch, s, tw, ramp);
+        if (!on) return;
+#pragma unroll
+        for (int n1 = 0; n1 < 16; ++n1) out[base + s + 8 * n1] = v[n1];
+    } else {
+        const int r = blockIdx.x * shift_lines<C>() + warp;
+        if (r >= rows) return;
+        const size_t base = ((size_t)blockIdx.y * rows + r) * C;
+        float2* line = scratch + warp * (tmp_line<C>() | 1);
+        for (int i = lane; i < C; i += 32) line[i] = in[base + i];
+        __syncwarp();
+        line_transform<C, -1>(line, tw, lane);
+        for (int i = lane; i < C; i += 32) line[i] = cmul(line[i], ramp[i]);
+        __syncwarp();
+        line_transform<C, +1>(line, tw, lane);
+        for (int i = lane; i < C; i += 32) out[base + i] = line[i];
     }
 }
 
-// Per strip of columns of every frame: FFT along the rows, the frame's
-// shift ramp, inverse FFT along the rows (in place). The ramp phase
-// -2 pi (f_r s_r + f_c s_c) is formed in FP64 and reduced before the
-// float32 sincos.
+// Columns, in place. 128 points: four neighbouring columns per warp (whole
+// 32-byte sectors) straight into registers; other sizes a strip of
+// kTmpWarps columns staged in shared memory, a warp per column.
 template <int R>
-__global__ void __launch_bounds__(32 * kTmpWarps) k_tmp_cols(float2* __restrict__ data, int cols,
-                                                             const float* __restrict__ shifts) {
-    constexpr int L = tmp_line<R>();
-    constexpr int P = L | 1;
-    extern __shared__ float2 tmp_cols_smem[];
-    float2* tile = tmp_cols_smem;
-    float2* tw = tile + kTmpWarps * P;
+__global__ void __launch_bounds__(32 * kTmpWarps) k_shift_cols(float2* __restrict__ data, int cols,
+                                                               const float* __restrict__ shifts) {
+    constexpr int P = tmp_line<R>() | 1;
+    extern __shared__ float2 tmp_smem[];
+    float2* tw = tmp_smem;
+    float2* ramp = tw + R;
+    float2* scratch = ramp + R;
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
-    const int frame = blockIdx.y;
-    const int c0 = blockIdx.x * kTmpWarps;
-    const int nc = min(kTmpWarps, cols - c0);
+    const int c0 = blockIdx.x * shift_lines<R>();
+    float2* d = data + (size_t)blockIdx.y * R * cols;
     fill_twiddles<R>(tw, tid, 32 * kTmpWarps);
-    float2* d = data + (size_t)frame * R * cols;
-    for (int e = tid; e < R * kTmpWarps; e += 32 * kTmpWarps) {
-        const int r = e / kTmpWarps;
-        const int c = e - r * kTmpWarps;
-        if (c < nc) tile[c * P + r] = d[(size_t)r * cols + c0 + c];
-    }
-    __syncthreads();
-    if (warp < nc) {
-        float2* line = tile + warp * P;
-        line_transform<R, -1>(line, tw, lane);
-        const double sr = (double)__ldg(shifts + 2 * frame);
-        const double sc = (double)__ldg(shifts + 2 * frame + 1);
-        const int c = c0 + warp;
-        const double fc = (double)(c < (cols + 1) / 2 ? c : c - cols) / (double)cols;
-        for (int r = lane; r < R; r += 32) {
-            const double fr = (double)(r < (R + 1) / 2 ? r : r - R) / (double)R;
-            double ph = -(fr * sr + fc * sc);  // in turns
-            ph -= rint(ph);
-            float s, co;
-            sincospif((float)(2.0 * ph), &s, &co);
-            line[r] = cmul(line[r], make_float2(co, s));
+    fill_ramp<R>(ramp, __ldg(shifts + 2 * blockIdx.y), tid, 32 * kTmpWarps);
+    if constexpr (R == 128) {
+        __syncthreads();
+        const int s = lane >> 2;  // lanes 4 s + j: column j of the warp's four
+        const int group = warp * 4 + (lane & 3);
+        const int c = c0 + group;
+        const bool on = c < cols;
+        float2* col = d + (on ? c : 0);
+        float2 v[16];
+#pragma unroll
+        for (int n1 = 0; n1 < 16; ++n1) v[n1] = col[(size_t)(s + 8 * n1) * cols];
+        // groups 4 float2 apart mod 16: the half-warp's 4 groups x 4 lanes meet no bank twice
+        shift_line128(v, scratch + group * (16 * kG8Pitch + 4), s, tw, ramp);
+        if (!on) return;
+#pragma unroll
+        for (int n1 = 0; n1 < 16; ++n1) col[(size_t)(s + 8 * n1) * cols] = v[n1];
+    } else {
+        const int nc = min(kTmpWarps, cols - c0);
+        for (int e = tid; e < R * kTmpWarps; e += 32 * kTmpWarps) {
+            const int r = e / kTmpWarps;
+            const int c = e - r * kTmpWarps;
+            if (c < nc) scratch[c * P + r] = d[(size_t)r * cols + c0 + c];
         }
-        __syncwarp();
-        line_transform<R, +1>(line, tw, lane);
-    }
-    __syncthreads();
-    for (int e = tid; e < R * kTmpWarps; e += 32 * kTmpWarps) {
-        const int r = e / kTmpWarps;
-        const int c = e - r * kTmpWarps;
-        if (c < nc) d[(size_t)r * cols + c0 + c] = tile[c * P + r];
+        __syncthreads();
+        if (warp < nc) {
+            float2* line = scratch + warp * P;
+            line_transform<R, -1>(line, tw, lane);
+            for (int r = lane; r < R; r += 32) line[r] = cmul(line[r], ramp[r]);
+            __syncwarp();
+            line_transform<R, +1>(line, tw, lane);
+        }
+        __syncthreads();
+        for (int e = tid; e < R * kTmpWarps; e += 32 * kTmpWarps) {
+            const int r = e / kTmpWarps;
+            const int c = e - r * kTmpWarps;
+            if (c < nc) d[(size_t)r * cols + c0 + c] = scratch[c * P + r];
+        }
     }
 }
 
-constexpr int kJoinBlocks = 64;   // overlap partial sums per frame
+constexpr int kJoinBlocks = 64;   // overlap partial sums per frame, at most
 constexpr int kJoinThreads = 256;
+
+// Blocks per frame of the overlap: 8 pixels per thread and more, so that the
+// block's reduction is small beside its reads (one pixel per thread took 30 us
+// at 256 frames of 128^2).
+static int overlap_blocks(long long n_pix) {
+    const long long b = (n_pix + 8 * kJoinThreads - 1) / (8 * kJoinThreads);
+    return b < kJoinBlocks ? (int)b : kJoinBlocks;
+}
+
+__device__ __forceinline__ double2 warp_sum(double2 v) {
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+    }
+    return v;
+}
 
 // partial[t][blk] = sum over this block's pixels of a_t conj(a_0), FP64.
 __global__ void __launch_bounds__(kJoinThreads) k_overlap_partial(const float2* __restrict__ a,
                                                                   long long n_pix,
                                                                   double2* __restrict__ partial) {
-    __shared__ double2 red[kJoinThreads];
+    __shared__ double2 red[kJoinThreads / 32];
     const int t = blockIdx.y;
     const float2* at = a + (size_t)t * n_pix;
-    double sr = 0.0, si = 0.0;
+    double2 sum = make_double2(0.0, 0.0);
     for (long long p = (long long)blockIdx.x * kJoinThreads + threadIdx.x; p < n_pix;
-         p += (long long)kJoinBlocks * kJoinThreads) {
+         p += (long long)gridDim.x * kJoinThreads) {
         const float2 v = at[p];
         const float2 r = a[p];
-        sr += (double)v.x * r.x + (double)v.y * r.y;
-        si += (double)v.y * r.x - (double)v.x * r.y;
+        sum.x += (double)v.x * r.x + (double)v.y * r.y;
+        sum.y += (double)v.y * r.x - (double)v.x * r.y;
     }
-    red[threadIdx.x] = make_double2(sr, si);
+    sum = warp_sum(sum);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
     __syncthreads();
-    for (int w = kJoinThreads / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) {
-            red[threadIdx.x].x += red[threadIdx.x + w].x;
-            red[threadIdx.x].y += red[threadIdx.x + w].y;
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kJoinThreads / 32; ++w) {
+            sum.x += red[w].x;
+            sum.y += red[w].y;
         }
-        __syncthreads();
+        partial[(size_t)t * gridDim.x + blockIdx.x] = sum;
     }
-    if (threadIdx.x == 0) partial[(size_t)t * kJoinBlocks + blockIdx.x] = red[0];
 }
 
-// rot[t] = exp(-i angle(overlap_t)) for t > 0, 1 for frame 0.
-__global__ void k_overlap_rotation(const double2* __restrict__ partial, int n_frames,
-                                   float2* __restrict__ rot) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// rot[t] = exp(-i angle(overlap_t)) for t > 0, 1 for frame 0; a warp per frame.
+__global__ void __launch_bounds__(128) k_overlap_rotation(const double2* __restrict__ partial,
+                                                          int n_blocks, int n_frames,
+                                                          float2* __restrict__ rot) {
+    const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
     if (t >= n_frames) return;
-    if (t == 0) {
-        rot[0] = make_float2(1.0f, 0.0f);
-        return;
+    double2 sum = make_double2(0.0, 0.0);
+    for (int b = lane; b < n_blocks; b += 32) {
+        const double2 v = partial[(size_t)t * n_blocks + b];
+        sum.x += v.x;
+        sum.y += v.y;
     }
-    double sr = 0.0, si = 0.0;
-    for (int b = 0; b < kJoinBlocks; ++b) {
-        sr += partial[(size_t)t * kJoinBlocks + b].x;
-        si += partial[(size_t)t * kJoinBlocks + b].y;
-    }
-    const double ang = atan2(si, sr);
-    rot[t] = make_float2((float)cos(ang), (float)-sin(ang));
+    sum = warp_sum(sum);
+    if (lane != 0) return;
+    const double ang = atan2(sum.y, sum.x);
+    rot[t] = t == 0 ? make_float2(1.0f, 0.0f) : make_float2((float)cos(ang), (float)-sin(ang));
 }
 
-// joined[p] = sum_t w_t rot_t a_t[p] (FP32, frames in order); the rotated
-// frames are written back when requested.
+// joined[p] = sum_t w_t rot_t a_t[p] in FP32; the rotated frames are written
+// back when requested. A block takes 32 pixels and its 8 warps every 8th
+// frame, the 8 sums added in order: a thread per pixel over all frames leaves
+// 64 blocks at 128^2 (52 us for 256 frames).
+constexpr int kJoinSlices = kJoinThreads / 32;
 __global__ void __launch_bounds__(kJoinThreads) k_join(float2* __restrict__ a,
                                                        const float* __restrict__ w,
                                                        const float2* __restrict__ rot,
                                                        int n_frames, long long n_pix,
                                                        float2* __restrict__ joined,
                                                        int write_back) {
-    const long long p = (long long)blockIdx.x * kJoinThreads + threadIdx.x;
-    if (p >= n_pix) return;
+    __shared__ float2 red[kJoinSlices][32];
+    const int lane = threadIdx.x & 31;
+    const int slice = threadIdx.x >> 5;
+    const long long p = (long long)blockIdx.x * 32 + lane;
     float sr = 0.0f, si = 0.0f;
-    for (int t = 0; t < n_frames; ++t) {
-        float2 v = a[(size_t)t * n_pix + p];
-        if (rot) v = cmul(v, __ldg(rot + t));
-        if (write_back) a[(size_t)t * n_pix + p] = v;
-        const float wt = __ldg(w + t);
-        sr = fmaf(wt, v.x, sr);
-        si = fmaf(wt, v.y, si);
+    if (p < n_pix) {
+#pragma unroll 4
+        for (int t = slice; t < n_frames; t += kJoinSlices) {
+            float2 v = a[(size_t)t * n_pix + p];
+            if (rot) v = cmul(v, __ldg(rot + t));
+            if (write_back) a[(size_t)t * n_pix + p] = v;
+            const float wt = __ldg(w + t);
+            sr = fmaf(wt, v.x, sr);
+            si = fmaf(wt, v.y, si);
+        }
+    }
+    red[slice][lane] = make_float2(sr, si);
+    __syncthreads();
+    if (slice != 0 || p >= n_pix) return;
+#pragma unroll
+    for (int k = 1; k < kJoinSlices; ++k) {
+        sr += red[k][lane].x;
+        si += red[k][lane].y;
     }
     joined[p] = make_float2(sr, si);
 }
 
-template <int C, int DIR>
-static void launch_rows(const float2* in, float2* out, int n_frames, int rows, float scale,
-                        cudaStream_t s) {
-    const size_t smem = sizeof(float2) * ((size_t)kTmpWarps * tmp_line<C>() + C);
-    cudaFuncSetAttribute(k_tmp_rows<C, DIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    { k_tmp_rows<C, DIR><<<dim3((rows + kTmpWarps - 1) / kTmpWarps, n_frames), 32 * kTmpWarps, smem, s>>>(
-        in, out, rows, scale); note_launch(); }
-}
-
-static int rows_pass(int cols, int dir, const float2* in, float2* out, int n_frames, int rows,
-                     float scale, cudaStream_t s) {
-    switch (cols) {
-#define QSSB_ROWS_CASE(n)                                                              \
-    case n:                                                                           \
-        if (dir < 0) launch_rows<n, -1>(in, out, n_frames, rows, scale, s);            \
-        else launch_rows<n, +1>(in, out, n_frames, rows, scale, s);                    \
-        break;
-        QSSB_ROWS_CASE(64)
-        QSSB_ROWS_CASE(128)
-        QSSB_ROWS_CASE(256)
-        QSSB_ROWS_CASE(512)
-        QSSB_ROWS_CASE(1024)
-#undef QSSB_ROWS_CASE
-        default:
-            return set_error(QSSB_ERR_UNSUPPORTED, "qssb_fourier_shift: sizes must be 64..1024, powers of two");
-    }
+template <int C>
+static int launch_rows(const float2* in, float2* out, int n_frames, int rows, const float* shifts,
+                       cudaStream_t s) {
+    constexpr int lines = shift_lines<C>();
+    CUDA_TRY(cudaFuncSetAttribute(k_shift_rows<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)shift_smem<C>()));
+    { k_shift_rows<C><<<dim3((rows + lines - 1) / lines, n_frames), 32 * kTmpWarps, shift_smem<C>(), s>>>(
+        in, out, rows, shifts); note_launch(); }
     CUDA_TRY(cudaGetLastError());
     return QSSB_OK;
 }
 
 template <int R>
 static int launch_cols(float2* data, int n_frames, int cols, const float* shifts, cudaStream_t s) {
-    const size_t smem = sizeof(float2) * ((size_t)kTmpWarps * (tmp_line<R>() | 1) + R);
-    CUDA_TRY(cudaFuncSetAttribute(k_tmp_cols<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    { k_tmp_cols<R><<<dim3((cols + kTmpWarps - 1) / kTmpWarps, n_frames), 32 * kTmpWarps, smem, s>>>(
+    constexpr int lines = shift_lines<R>();
+    CUDA_TRY(cudaFuncSetAttribute(k_shift_cols<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)shift_smem<R>()));
+    { k_shift_cols<R><<<dim3((cols + lines - 1) / lines, n_frames), 32 * kTmpWarps, shift_smem<R>(), s>>>(
         data, cols, shifts); note_launch(); }
     CUDA_TRY(cudaGetLastError());
     return QSSB_OK;
@@ -248,18 +334,24 @@ extern "C" int qssb_fourier_shift(const float* in, float* out, int32_t n_frames,
     if (!tmp_size_ok(rows) || !tmp_size_ok(cols))
         return set_error(QSSB_ERR_UNSUPPORTED, "qssb_fourier_shift: sizes must be 64..1024, powers of two");
     cudaStream_t s = (cudaStream_t)stream;
+    auto* i = reinterpret_cast<const float2*>(in);
     auto* o = reinterpret_cast<float2*>(out);
-    int rc = rows_pass(cols, -1, reinterpret_cast<const float2*>(in), o, n_frames, rows, 1.0f, s);
-    if (rc) return rc;
-    switch (rows) {
-        case 64: rc = launch_cols<64>(o, n_frames, cols, shifts, s); break;
-        case 128: rc = launch_cols<128>(o, n_frames, cols, shifts, s); break;
-        case 256: rc = launch_cols<256>(o, n_frames, cols, shifts, s); break;
-        case 512: rc = launch_cols<512>(o, n_frames, cols, shifts, s); break;
-        default: rc = launch_cols<1024>(o, n_frames, cols, shifts, s); break;
+    int rc;
+    switch (cols) {
+        case 64: rc = launch_rows<64>(i, o, n_frames, rows, shifts, s); break;
+        case 128: rc = launch_rows<128>(i, o, n_frames, rows, shifts, s); break;
+        case 256: rc = launch_rows<256>(i, o, n_frames, rows, shifts, s); break;
+        case 512: rc = launch_rows<512>(i, o, n_frames, rows, shifts, s); break;
+        default: rc = launch_rows<1024>(i, o, n_frames, rows, shifts, s); break;
     }
     if (rc) return rc;
-    return rows_pass(cols, +1, o, o, n_frames, rows, 1.0f / ((float)rows * (float)cols), s);
+    switch (rows) {
+        case 64: return launch_cols<64>(o, n_frames, cols, shifts, s);
+        case 128: return launch_cols<128>(o, n_frames, cols, shifts, s);
+        case 256: return launch_cols<256>(o, n_frames, cols, shifts, s);
+        case 512: return launch_cols<512>(o, n_frames, cols, shifts, s);
+        default: return launch_cols<1024>(o, n_frames, cols, shifts, s);
+    }
 }
 
 extern "C" int qssb_join_workspace_bytes(int32_t n_frames, size_t* bytes) {
@@ -292,12 +384,13 @@ extern "C" int qssb_join_object_waves(float* frames, const float* weights, int32
         auto* partial = static_cast<double2*>(workspace);
         const size_t part = (sizeof(double2) * (size_t)n_frames * kJoinBlocks + 255) & ~(size_t)255;
         rot = reinterpret_cast<float2*>(static_cast<char*>(workspace) + part);
-        { k_overlap_partial<<<dim3(kJoinBlocks, n_frames), kJoinThreads, 0, s>>>(a, n_pix, partial); note_launch(); }
+        const int n_blocks = overlap_blocks(n_pix);
+        { k_overlap_partial<<<dim3(n_blocks, n_frames), kJoinThreads, 0, s>>>(a, n_pix, partial); note_launch(); }
         CUDA_TRY(cudaGetLastError());
-        { k_overlap_rotation<<<(n_frames + 127) / 128, 128, 0, s>>>(partial, n_frames, rot); note_launch(); }
+        { k_overlap_rotation<<<(n_frames + 3) / 4, 128, 0, s>>>(partial, n_blocks, n_frames, rot); note_launch(); }
         CUDA_TRY(cudaGetLastError());
     }
-    const long long blocks = (n_pix + kJoinThreads - 1) / kJoinThreads;
+    const long long blocks = (n_pix + 31) / 32;
     if (blocks > 0x7fffffffLL) return set_error(QSSB_ERR_INVALID, "qssb_join_object_waves: too many pixels");
     { k_join<<<(unsigned)blocks, kJoinThreads, 0, s>>>(a, weights, rot, n_frames, n_pix,
                                                      reinterpret_cast<float2*>(joined), write_back); note_launch(); }

@@ -143,3 +143,18 @@ def test_time_series_through_ssb_sessions():
     assert avg.object_wave.shape == (128, 128)
     for s in sessions:
         s.close()
+
+
+@pytest.mark.parametrize("shape", [(64, 128), (128, 64), (128, 1024)])
+@pytest.mark.parametrize("n", [1, 8, 9, 67])
+def test_join_slices_and_strips(shape, n):
+    """Frame counts around the join's 8 slices, columns and rows fewer than,
+    equal to and more than a block's 32 lines; float32 sums, 3e-6 as above."""
+    rng = np.random.default_rng(n + shape[0])
+    waves = rng.standard_normal((n, *shape)) + 1j * rng.standard_normal((n, *shape))
+    shifts = rng.uniform(-6.0, 6.0, (n, 2))
+    for ref in ("first", "none"):
+        want, _ = to.join_object_waves(waves, shifts, None, ref)
+        got = join_object_waves(torch.as_tensor(waves.astype(np.complex64), device=DEV),
+                                shifts=shifts, phase_reference=ref)
+        assert np.abs(got.object_wave.cpu().numpy() - want).max() < 3e-6 * np.abs(waves).max()
