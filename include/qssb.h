@@ -113,6 +113,21 @@ int64_t qssb_kernel_launches(void);
 int qssb_mean_dp_u64(const uint16_t* counts, int64_t n_frames, int32_t det_pixels,
                      uint64_t* sums, float* mean_dp, void* stream);
 
+/* The padding of a scan to its square native size (backend.py:229-269)
+ * without writing the padded counts. qssb_pad_fill: fill[k] =
+ * floor(sums[k] / n_frames) as u16, the pattern of every border frame, and
+ * padded_sums[k] = sums[k] + (n_padded - n_frames) * fill[k], the sums of the
+ * padded scan. qssb_pad_columns: gathered columns [n_bf][rows][cols] to
+ * out [n_bf][out_rows][out_cols] with the scan at (top, left) and
+ * fill[bf_linear[b]] around it (out_cols a multiple of 8, out 16-byte
+ * aligned, not overlapping columns). */
+int qssb_pad_fill(const uint64_t* sums, int32_t det_pixels, int64_t n_frames, int64_t n_padded,
+                  uint16_t* fill, uint64_t* padded_sums, void* stream);
+int qssb_pad_columns(const uint16_t* columns, int32_t n_bf, int32_t rows, int32_t cols,
+                     const uint16_t* fill, const int32_t* bf_linear, int32_t det_pixels,
+                     int32_t out_rows, int32_t out_cols, int32_t top, int32_t left, uint16_t* out,
+                     void* stream);
+
 /* BF-column gather: columns[b][f] = counts[f][bf_linear[b]] (exact u16).
  * Replaces the fancy-index + transpose of _extract_gqk (backend.py:561-572).
  * bf_linear: device int32 [n_bf], each in [0, det_pixels). */

@@ -121,6 +121,9 @@ SIGNATURES = {
     "qssb_version": (ctypes.c_int, []),
     "qssb_last_error": (ctypes.c_char_p, []),
     "qssb_mean_dp_u64": (ctypes.c_int, [_P, _I64, _I32, _P, _P, _P]),
+    "qssb_pad_fill": (ctypes.c_int, [_P, _I32, _I64, _I64, _P, _P, _P]),
+    "qssb_pad_columns": (ctypes.c_int, [_P, _I32, _I32, _I32, _P, _P, _I32, _I32, _I32, _I32, _I32,
+                                        _P, _P]),
     "qssb_gather_bf_columns": (ctypes.c_int, [_P, _I64, _I32, _P, _I32, _P, _P]),
     "qssb_gather_bf_columns_2d": (ctypes.c_int, [_P, _I64, _I32, _I32, _P, _I32, _P, _P]),
     "qssb_gather_bf_columns_2d_ex": (ctypes.c_int, [_P, _I64, _I32, _I32, _P, _I32, _P, _I32, _P]),

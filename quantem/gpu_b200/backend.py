@@ -169,7 +169,8 @@ class B200SSBBackend:
             counts = counts.reshape(scan_shape[0], scan_shape[1], counts.shape[1], counts.shape[2])
         elif counts.ndim != 4:
             raise ValueError("data must be 3D or 4D.")
-        counts = self._pad_or_crop(counts)
+        counts, scan_gpts = self._crop(counts)
+        rows, cols = int(counts.shape[0]), int(counts.shape[1])
         if isinstance(scan_sampling, (int, float)):
             scan_sampling = (float(scan_sampling), float(scan_sampling))
         self.energy = energy
@@ -182,7 +183,6 @@ class B200SSBBackend:
         self._rotation_angle_rad = math.radians(rotation_angle_deg)
         self.gqk_storage = gqk_storage
         self._flags = QSSB_FLAG_CHI_FP64 if chi_fp64 else 0
-        scan_gpts = (int(counts.shape[0]), int(counts.shape[1]))
         det_gpts = (int(counts.shape[2]), int(counts.shape[3]))
         if scan_gpts[0] not in NATIVE_SCAN_SIZES:
             raise NotImplementedError(
@@ -191,8 +191,12 @@ class B200SSBBackend:
             )
         self.wavelength = electron_wavelength_angstrom(energy)
         n_frames = scan_gpts[0] * scan_gpts[1]
-        # (a3) exact u64 frame sums on the GPU
+        # (a3) exact u64 frame sums on the GPU, of the padded scan where it is
+        # smaller than its native size
         sums_dev, _ = ops.mean_dp_u64(counts, want_mean=False)
+        fill = None
+        if (rows, cols) != scan_gpts:
+            fill, sums_dev = ops.pad_fill(sums_dev, rows * cols, n_frames)
         self._detected_radius_px = None
         sums_host = None
         if det_sampling is None:
@@ -254,6 +258,9 @@ class B200SSBBackend:
         self._cached_rotation = self._rotation_angle_rad
         # (a6) gather + Hermitian scan FFT; dc exact from the integer sums
         columns = ops.gather_bf_columns(counts, self._bf_linear, validate=False)
+        if fill is not None:
+            columns = ops.pad_columns(columns, (rows, cols), fill, self._bf_linear, scan_gpts[0],
+                                      (scan_gpts[0] - rows) // 2, (scan_gpts[1] - cols) // 2)
         self.G_qk = ops.scan_fft_half(columns, scan_gpts)
         del columns
         self._workspace = ops.Workspace(self.device)
@@ -269,27 +276,22 @@ class B200SSBBackend:
         self.timings = {"prepare_s": time.perf_counter() - t0}
 
     # ------------------------------------------------------------ preparation
-    def _pad_or_crop(self, counts: torch.Tensor) -> torch.Tensor:
-        """Reference padding rule (backend.py:229-269) on the device."""
+    @staticmethod
+    def _crop(counts: torch.Tensor) -> tuple[torch.Tensor, tuple[int, int]]:
+        """The counts with the axes longer than the reference's square target
+        cropped to its centre (backend.py:229-269), and the scan's size after
+        the rule (its border, where an axis is shorter, is added to the BF
+        columns alone)."""
         h, w = int(counts.shape[0]), int(counts.shape[1])
         target = pad_target(h, w)
         if target is None:
-            return counts
+            return counts, (h, w)
         t = target[0]
         if h > t or w > t:
             r0 = max(0, (h - t) // 2)
             c0 = max(0, (w - t) // 2)
             counts = counts[r0:r0 + min(t, h), c0:c0 + min(t, w)].contiguous()
-            h, w = int(counts.shape[0]), int(counts.shape[1])
-        if h < t or w < t:
-            sums, _ = ops.mean_dp_u64(counts, want_mean=False)
-            n = h * w
-            fill = (sums.cpu().numpy().view(np.uint64).astype(np.float64) / n).astype(np.uint16)
-            padded = torch.as_tensor(fill, device=self.device).expand(t, t, *fill.shape).contiguous()
-            top, left = (t - h) // 2, (t - w) // 2
-            padded[top:top + h, left:left + w] = counts
-            counts = padded
-        return counts
+        return counts, (t, t)
 
     # ---------------------------------------------------------------- helpers
     def _k_step(self) -> tuple[float, float]:

@@ -149,6 +149,33 @@ def mean_dp_u64(counts: torch.Tensor, want_mean: bool = True
     return sums, mean
 
 
+def pad_fill(sums: torch.Tensor, n_frames: int, n_padded: int) -> tuple[torch.Tensor, torch.Tensor]:
+    """(fill u16, padded sums as int64, both of ``sums``'s shape) of a scan of
+    ``n_frames`` padded to ``n_padded`` by frames of its floored mean pattern."""
+    _require_cuda(sums, "sums", torch.int64)
+    fill = torch.empty(sums.shape, dtype=torch.uint16, device=sums.device)
+    padded = torch.empty_like(sums)
+    _call("qssb_pad_fill", sums.device, _ptr(sums), sums.numel(), int(n_frames), int(n_padded),
+          _ptr(fill), _ptr(padded), _stream(sums))
+    return fill, padded
+
+
+def pad_columns(columns: torch.Tensor, scan_shape: tuple[int, int], fill: torch.Tensor,
+                bf_linear: torch.Tensor, side: int, top: int, left: int) -> torch.Tensor:
+    """Gathered columns [n_bf, rows * cols] with their border: u16 [n_bf, side * side]."""
+    _require_cuda(columns, "columns", torch.uint16)
+    _require_cuda(fill, "fill", torch.uint16)
+    _require_cuda(bf_linear, "bf_linear", torch.int32)
+    n_bf = int(columns.shape[0])
+    rows, cols = (int(v) for v in scan_shape)
+    if columns.numel() != n_bf * rows * cols or bf_linear.numel() != n_bf:
+        raise ValueError("columns must be [n_bf, rows * cols] with one index per column")
+    out = torch.empty((n_bf, side * side), dtype=torch.uint16, device=columns.device)
+    _call("qssb_pad_columns", columns.device, _ptr(columns), n_bf, rows, cols, _ptr(fill),
+          _ptr(bf_linear), fill.numel(), side, side, int(top), int(left), _ptr(out), _stream(columns))
+    return out
+
+
 def mean_from_sums(sums_u64, n_frames: int):
     """float32(sum) / n_frames with IEEE rounding: the kernel's mean, on the host."""
     import numpy as np
