@@ -585,6 +585,13 @@ int qssb_adam(float* w, float* m, float* v, const float* grad, int64_t n, float 
  * first_step: the step count when this cosine run began). */
 int qssb_adam_schedule(float* hyper, int32_t* step, int32_t first_step, int32_t total_steps,
                        float lr0, float beta1, float beta2, void* stream);
+/* The same for n_tensors (at most 8) parameter tensors in one launch: host
+ * arrays of device pointers, element counts and weight decays; w_bf16[i] may
+ * be NULL. With hyper (device {lr, c1, c2}, or NULL) lr and step are not read. */
+int qssb_adam_multi(int32_t n_tensors, float* const* w, float* const* m, float* const* v,
+                    const float* const* grad, const int64_t* n, const float* weight_decay,
+                    void* const* w_bf16, float lr, float beta1, float beta2, float eps,
+                    int32_t step, const float* hyper, void* stream);
 /* qssb_adam with the learning rate and bias corrections read from hyper
  * (device {lr, c1, c2}, as qssb_adam_schedule writes them). */
 int qssb_adam_dev(float* w, float* m, float* v, const float* grad, int64_t n, const float* hyper,

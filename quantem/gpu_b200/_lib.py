@@ -167,6 +167,8 @@ SIGNATURES = {
                                       _P, _P, _P, _P]),
     "qssb_adam": (ctypes.c_int, [_P, _P, _P, _P, _I64, ctypes.c_float, ctypes.c_float,
                                  ctypes.c_float, ctypes.c_float, ctypes.c_float, _I32, _P, _P]),
+    "qssb_adam_multi": (ctypes.c_int, [_I32, _P, _P, _P, _P, _P, _P, _P, ctypes.c_float,
+                                       ctypes.c_float, ctypes.c_float, ctypes.c_float, _I32, _P, _P]),
     "qssb_adam_schedule": (ctypes.c_int, [_P, _P, _I32, _I32, ctypes.c_float, ctypes.c_float,
                                           ctypes.c_float, _P]),
     "qssb_adam_dev": (ctypes.c_int, [_P, _P, _P, _P, _I64, _P, ctypes.c_float, ctypes.c_float,

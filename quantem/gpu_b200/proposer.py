@@ -418,18 +418,16 @@ class MLP:
         self.t += 1
         params = self.w + self.b
         grads = bf["gw"] + bf["gb"]
-        for j, (p, gr) in enumerate(zip(params, grads)):
-            wbf = self.w_bf[j] if j < 4 else None
-            if hyper is None:
-                _call("qssb_adam", dev, _ptr(p), _ptr(self.m[j]), _ptr(self.v[j]), _ptr(gr),
-                      p.numel(), ctypes.c_float(lr), ctypes.c_float(ADAM_BETAS[0]),
-                      ctypes.c_float(ADAM_BETAS[1]), ctypes.c_float(1e-8),
-                      ctypes.c_float(wd if j < 4 else 0.0), self.t, _ptr(wbf), _stream(dev))
-            else:
-                _call("qssb_adam_dev", dev, _ptr(p), _ptr(self.m[j]), _ptr(self.v[j]), _ptr(gr),
-                      p.numel(), _ptr(hyper), ctypes.c_float(ADAM_BETAS[0]),
-                      ctypes.c_float(ADAM_BETAS[1]), ctypes.c_float(1e-8),
-                      ctypes.c_float(wd if j < 4 else 0.0), _ptr(wbf), _stream(dev))
+        copies = self.w_bf + [None] * 4
+
+        def pointers(tensors):
+            return (ctypes.c_void_p * 8)(*(0 if t is None else t.data_ptr() for t in tensors))
+
+        _call("qssb_adam_multi", dev, 8, pointers(params), pointers(self.m), pointers(self.v),
+              pointers(grads), (ctypes.c_int64 * 8)(*(p.numel() for p in params)),
+              (ctypes.c_float * 8)(wd, wd, wd, wd, 0.0, 0.0, 0.0, 0.0), pointers(copies),
+              ctypes.c_float(lr), ctypes.c_float(ADAM_BETAS[0]), ctypes.c_float(ADAM_BETAS[1]),
+              ctypes.c_float(1e-8), self.t, _ptr(hyper), _stream(dev))
         return bf["loss"]
 
     def predict(self, x: torch.Tensor) -> np.ndarray:

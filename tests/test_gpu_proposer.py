@@ -280,3 +280,37 @@ def test_forward_model_features_match_simulated_scans():
             be.close()
         assert min(cos_all) >= lo, (peak, cos_all)
         assert np.mean(cos_all) >= mean, (peak, np.mean(cos_all))
+
+
+def test_adam_multi_takes_remainders_and_unaligned_tensors():
+    """One launch over tensors around the 4096-element block and off 16-byte
+    alignment, with and without the BF16 copy; a dozen float32 operations per
+    element, each within 2^-24: 2e-6 of the update's scale."""
+    sizes = [1, 4095, 4096, 4097, 9000]
+    g = torch.Generator(device=DEV).manual_seed(3)
+    rnd = lambda n, off: torch.randn(n + off, device=DEV, generator=g)[off:]  # noqa: E731
+    offs = [0, 0, 0, 0, 1]
+    w, m, grad = ([rnd(n, o) for n, o in zip(sizes, offs)] for _ in range(3))
+    v = [rnd(n, o).square() for n, o in zip(sizes, offs)]
+    copy = [torch.empty(n, dtype=torch.bfloat16, device=DEV) if i % 2 else None
+            for i, n in enumerate(sizes)]
+    wd = [0.1, 0.0, 0.2, 0.0, 0.3]
+    lr, b1, b2, eps, step, k = 1e-2, 0.9, 0.999, 1e-8, 3, len(sizes)
+    want = []
+    for i in range(k):
+        mi = b1 * m[i].double() + (1 - b1) * grad[i].double()
+        vi = b2 * v[i].double() + (1 - b2) * grad[i].double() ** 2
+        upd = (mi / (1 - b1 ** step)) / ((vi / (1 - b2 ** step)).sqrt() + eps) + wd[i] * w[i].double()
+        want.append((w[i].double() - lr * upd, mi, vi))
+    ptrs = lambda ts: (ctypes.c_void_p * k)(*(0 if t is None else t.data_ptr() for t in ts))  # noqa: E731
+    torch.cuda.synchronize()
+    _lib.check(_lib.load().qssb_adam_multi(
+        k, ptrs(w), ptrs(m), ptrs(v), ptrs(grad), (ctypes.c_int64 * k)(*sizes),
+        (ctypes.c_float * k)(*wd), ptrs(copy), ctypes.c_float(lr), ctypes.c_float(b1),
+        ctypes.c_float(b2), ctypes.c_float(eps), step, None, None))
+    torch.cuda.synchronize()
+    for i in range(k):
+        for got, ref in zip((w[i], m[i], v[i]), want[i]):
+            torch.testing.assert_close(got.double(), ref, rtol=2e-6, atol=2e-6)
+        if copy[i] is not None:
+            torch.testing.assert_close(copy[i], w[i].to(torch.bfloat16), rtol=0, atol=0)
