@@ -11,8 +11,8 @@
 // 8k+j in bit j); the last block holds the rest rounded down to 8 elements;
 // the remaining < 8 elements follow raw.
 //
-// Decode: one CTA per chunk. Thread 0 walks the block chain (every offset
-// checked against the chunk's end); each warp decodes a block's LZ4
+// Decode: one CTA per chunk. Each warp walks the block chain (every offset
+// checked against the chunk's end) and decodes its blocks' LZ4
 // sequences into shared memory (every lane parses the token stream through
 // L1, all lanes copy literals and matches - a match byte j reads
 // out[op - off + j mod off], so overlapping matches need no serial copy) and
@@ -57,6 +57,74 @@ __device__ __forceinline__ uint64_t transpose8(uint64_t x) {
     return x;
 }
 
+// Four bytes at any byte position of a 4-aligned shared buffer. The second
+// word of an aligned position is read too (inside the kernel's shared memory
+// in every use) and shifted out.
+__device__ __forceinline__ uint32_t rd32(const uint8_t* base, int pos) {
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(base) + (pos >> 2);
+    return __funnelshift_r(w[0], w[1], 8 * (pos & 3));
+}
+
+// out[op + j] = out[op - off + j], j < ml, by the whole warp, as if byte by
+// byte (off < ml repeats the last off bytes). Up to 32 bytes in one step.
+// Longer: the output has period off, so it may be read from any multiple of
+// off back that lies behind op - off; bytes fill the first multiple D >= 128,
+// then words copy from D back, 128 bytes a step and, once D has doubled to
+// 512, 512 a step (the runs of zero planes: 8 KB in ~25 steps).
+__device__ __forceinline__ void copy_match(uint8_t* out, int op, int off, int ml, int lane) {
+    // lane mod off: (lane + 1/2) / off is never within 1/64 of an integer
+    const int r0 = off > 31 ? lane : lane - off * (int)__fdividef((float)lane + 0.5f, (float)off);
+    if (ml <= 32) {
+        if (lane < ml) out[op + lane] = out[op - off + r0];
+        return;
+    }
+    int d = off;
+    if (d < 128) d *= (127 + off) / off;
+    const int n0 = min(ml, (off < 128 ? d : 0) + ((4 - ((op + (off < 128 ? d : 0)) & 3)) & 3));
+    if (off < 32) {
+        int r = r0;
+        const int step = 32 % off;
+        for (int j = lane; j < n0; j += 32) {
+            out[op + j] = out[op - off + r];
+            r += step;
+            if (r >= off) r -= off;
+        }
+    } else {  // 32 <= off: a step reads behind what it writes
+        for (int j0 = 0; j0 < n0; j0 += 32) {
+            if (j0 + lane < n0) out[op + j0 + lane] = out[op - off + j0 + lane];
+            __syncwarp();
+        }
+    }
+    __syncwarp();
+    int p = op + n0;  // a multiple of 4 while words remain
+    int words = (ml - n0) >> 2;
+    while (words > 0) {
+        while (d < 512 && p - 2 * d >= op - off) d *= 2;
+        if (d >= 512) {
+            uint32_t w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (lane + 32 * u < words) w[u] = rd32(out, p - d + 4 * (lane + 32 * u));
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (lane + 32 * u < words)
+                    *reinterpret_cast<uint32_t*>(out + p + 4 * (lane + 32 * u)) = w[u];
+            const int n = min(words, 128);
+            p += 4 * n;
+            words -= n;
+        } else {
+            if (lane < words)
+                *reinterpret_cast<uint32_t*>(out + p + 4 * lane) = rd32(out, p - d + 4 * lane);
+            const int n = min(words, 32);
+            p += 4 * n;
+            words -= n;
+        }
+        __syncwarp();
+    }
+    const int rest = op + ml - p;
+    if (lane < rest) out[p + lane] = out[p - d + lane];
+}
+
 // Decode one LZ4 block from in[0, csz) (global memory, read through L1) into
 // out[0, cap) (shared memory) by the whole warp. Every lane parses the token
 // stream itself (the same bytes: broadcast reads, uniform control flow, no
@@ -78,6 +146,7 @@ __device__ bool lz4_block_warp(const uint8_t* __restrict__ in, int csz, uint8_t*
             } while (b == 255 && lit <= cap);
         }
         if (lit > cap - op || lit > csz - ip) return false;
+#pragma unroll 4
         for (int j = lane; j < lit; j += 32) out[op + j] = __ldg(in + ip + j);
         ip += lit;
         op += lit;
@@ -99,28 +168,74 @@ __device__ bool lz4_block_warp(const uint8_t* __restrict__ in, int csz, uint8_t*
         }
         if (off == 0 || off > op || ml > cap - op) return false;
         __syncwarp();  // literals (and earlier matches) visible to the match reads
-        if (off >= ml) {  // no self-overlap: a plain copy
-            for (int j = lane; j < ml; j += 32) out[op + j] = out[op - off + j];
-        } else {
-            // out[op + j] = out[op - off + (j mod off)]: reads only bytes before op
-            int r = lane % off;
-            const int step = 32 % off;
-            for (int j = lane; j < ml; j += 32) {
-                out[op + j] = out[op - off + r];
-                r += step;
-                if (r >= off) r -= off;
-            }
-        }
+        copy_match(out, op, off, ml, lane);
         op += ml;
         __syncwarp();
     }
     return false;
 }
 
+// Bytes g of the eight words w, g = 0..3, as 8-byte values m[g] (byte b from w[b]).
+__device__ __forceinline__ void byte_columns(const uint32_t* w, uint64_t* m) {
+    uint32_t h[2][4];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const uint32_t* x = w + 4 * k;
+        const uint32_t a = __byte_perm(x[0], x[1], 0x5140), b = __byte_perm(x[2], x[3], 0x5140);
+        const uint32_t c = __byte_perm(x[0], x[1], 0x7362), d = __byte_perm(x[2], x[3], 0x7362);
+        h[k][0] = __byte_perm(a, b, 0x5410);
+        h[k][1] = __byte_perm(a, b, 0x7632);
+        h[k][2] = __byte_perm(c, d, 0x5410);
+        h[k][3] = __byte_perm(c, d, 0x7632);
+    }
+#pragma unroll
+    for (int g = 0; g < 4; ++g) m[g] = (uint64_t)h[0][g] | ((uint64_t)h[1][g] << 32);
+}
+
+// Eight u16 elements from their low and high bytes.
+__device__ __forceinline__ uint4 join_bytes(uint64_t lo, uint64_t hi) {
+    const uint32_t l0 = (uint32_t)lo, l1 = (uint32_t)(lo >> 32);
+    const uint32_t h0 = (uint32_t)hi, h1 = (uint32_t)(hi >> 32);
+    return make_uint4(__byte_perm(l0, h0, 0x5140), __byte_perm(l0, h0, 0x7362),
+                      __byte_perm(l1, h1, 0x5140), __byte_perm(l1, h1, 0x7362));
+}
+
 // Bit-unshuffle cnt (a multiple of 8) elements from a block's planes into dst.
+// wide: dst is 32-byte aligned; a lane then takes a word of every plane (32
+// elements, the high planes skipped where they are zero) and stores whole
+// 32-byte sectors. Otherwise (and where a plane is not whole words) a byte of
+// every plane, 8 elements.
 __device__ __forceinline__ void unshuffle_store(const uint8_t* planes, int cnt, uint16_t* dst,
-                                                bool vec, int lane) {
+                                                bool vec, bool wide, int lane) {
     const int P = cnt / 8;
+    if (wide && (P & 3) == 0) {
+        const uint32_t* words = reinterpret_cast<const uint32_t*>(planes);
+        for (int q = lane; q < P / 4; q += 32) {
+            uint32_t w[16];
+            uint32_t high = 0;
+#pragma unroll
+            for (int b = 0; b < 16; ++b) {
+                w[b] = words[b * (P / 4) + q];
+                if (b >= 8) high |= w[b];
+            }
+            uint64_t lo[4], hi[4] = {0, 0, 0, 0};
+            byte_columns(w, lo);
+            if (high) {
+                byte_columns(w + 8, hi);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) hi[g] = transpose8(hi[g]);
+            }
+#pragma unroll
+            for (int g = 0; g < 4; g += 2) {
+                const uint4 a = join_bytes(transpose8(lo[g]), hi[g]);
+                const uint4 b = join_bytes(transpose8(lo[g + 1]), hi[g + 1]);
+                asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                             :: "l"(dst + 32 * q + 8 * g), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+                                "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+            }
+        }
+        return;
+    }
     for (int p = lane; p < P; p += 32) {
         uint64_t lo = 0, hi = 0;
 #pragma unroll
@@ -128,44 +243,36 @@ __device__ __forceinline__ void unshuffle_store(const uint8_t* planes, int cnt, 
             lo |= (uint64_t)planes[b * P + p] << (8 * b);
             hi |= (uint64_t)planes[(8 + b) * P + p] << (8 * b);
         }
-        lo = transpose8(lo);  // byte j: bits 0..7 of element 8p + j
-        hi = transpose8(hi);  // byte j: bits 8..15
-        uint32_t w[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint32_t e0 = (uint32_t)((lo >> (16 * q)) & 0xff) | ((uint32_t)((hi >> (16 * q)) & 0xff) << 8);
-            const uint32_t e1 = (uint32_t)((lo >> (16 * q + 8)) & 0xff) | ((uint32_t)((hi >> (16 * q + 8)) & 0xff) << 8);
-            w[q] = e0 | (e1 << 16);
-        }
+        // transposed: byte j of lo (hi) holds bits 0..7 (8..15) of element 8p + j
+        const uint4 w = join_bytes(transpose8(lo), transpose8(hi));
         uint16_t* o = dst + 8 * p;
         if (vec) {
-            *reinterpret_cast<uint4*>(o) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(o) = w;
         } else {
+            const uint32_t e[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                o[2 * q] = (uint16_t)(w[q] & 0xffff);
-                o[2 * q + 1] = (uint16_t)(w[q] >> 16);
+                o[2 * q] = (uint16_t)(e[q] & 0xffff);
+                o[2 * q + 1] = (uint16_t)(e[q] >> 16);
             }
         }
     }
 }
 
-struct DecSmem {
-    int start[kMaxBlocks];  // block's LZ4 data offset within the chunk
-    int size[kMaxBlocks];
-    int tail_at;            // raw leftover elements' offset
-    int status;
-};
-
-__global__ void __launch_bounds__(32 * kDecWarps) k_decode_bslz4_u16(
+// W warps per chunk, which share nothing: each walks the block chain itself
+// (every lane reads the same words, prefetched into L1), first to the end to
+// check it, then along the blocks it takes. W = 1 where the chunks fill the
+// chip: a frame's blocks differ widely in cost, and the warps of a larger CTA
+// hold their shared memory until its slowest is done.
+template <int W>
+__global__ void __launch_bounds__(32 * W) k_decode_bslz4_u16(
     const uint8_t* __restrict__ comp, long long comp_bytes, const long long* __restrict__ offsets,
     int n_chunks, long long chunk_bytes, uint16_t* __restrict__ out, int* __restrict__ status) {
-    extern __shared__ uint4 dec_smem4[];
-    uint8_t* wbuf = reinterpret_cast<uint8_t*>(dec_smem4);  // per warp: one decoded block
-    __shared__ DecSmem sh;
+    __shared__ uint4 planes4[W * kBlockBytes / 16 + 1];  // + a word that unaligned reads may touch
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
+    uint8_t* planes = reinterpret_cast<uint8_t*>(planes4) + (size_t)warp * kBlockBytes;
     const int c = blockIdx.x;
     const long long n_elem = chunk_bytes / 2;
     const long long n8 = n_elem & ~7LL;
@@ -174,62 +281,61 @@ __global__ void __launch_bounds__(32 * kDecWarps) k_decode_bslz4_u16(
     const long long c1 = c + 1 < n_chunks ? offsets[c + 1] : comp_bytes;
     const uint8_t* ch = comp + c0;
     const long long len = c1 - c0;
-    if (c0 >= 0 && c1 <= comp_bytes) {
-        // the chunk's bytes into L1 (one prefetch per 128-byte line) before the
-        // serial block-chain walk and the parses read them
-        for (long long i = (long long)tid * 128; i < len; i += 128LL * 32 * kDecWarps)
+    int st = kStOk;
+    if (c0 < 0 || c1 > comp_bytes || len < 12) {
+        st = kStHeader;
+    } else {
+        // the chunk's bytes into L1 (one prefetch per 128-byte line)
+        for (long long i = (long long)tid * 128; i < len; i += 128LL * 32 * W)
             asm volatile("prefetch.global.L1 [%0];" ::"l"(ch + i));
+        unsigned long long total = 0;
+        for (int i = 0; i < 8; ++i) total = (total << 8) | ch[i];
+        if ((long long)total != chunk_bytes || be32(ch + 8) != (uint32_t)kBlockBytes) st = kStHeader;
     }
-    __syncthreads();
-    if (tid == 0) {
-        int st = kStOk;
-        if (c0 < 0 || c1 > comp_bytes || len < 12) {
-            st = kStHeader;
-        } else {
-            unsigned long long total = 0;
-            for (int i = 0; i < 8; ++i) total = (total << 8) | ch[i];
-            if ((long long)total != chunk_bytes || be32(ch + 8) != (uint32_t)kBlockBytes) st = kStHeader;
-        }
-        long long pos = 12;
-        for (int i = 0; i < n_blocks && st == kStOk; ++i) {
-            if (pos + 4 > len) { st = kStChain; break; }
-            const long long csz = be32(ch + pos);
-            if (csz > kLz4Bound || pos + 4 + csz > len) { st = kStChain; break; }
-            sh.start[i] = (int)(pos + 4);
-            sh.size[i] = (int)csz;
-            pos += 4 + csz;
-        }
-        if (st == kStOk && pos + (n_elem - n8) * 2 > len) st = kStChain;
-        sh.tail_at = (int)pos;
-        sh.status = st;
-        if (status) status[c] = st;  // blocks that fail raise it below
+    long long pos = 12;
+    for (int i = 0; i < n_blocks && st == kStOk; ++i) {
+        if (pos + 4 > len) { st = kStChain; break; }
+        const long long csz = be32(ch + pos);
+        if (csz > kLz4Bound || pos + 4 + csz > len) { st = kStChain; break; }
+        pos += 4 + csz;
     }
-    __syncthreads();
+    if (st == kStOk && pos + (n_elem - n8) * 2 > len) st = kStChain;
     uint16_t* frame = out + (size_t)c * n_elem;
-    const bool vec = (n_elem & 7) == 0 && ((uintptr_t)out & 15u) == 0;
-    if (sh.status != kStOk) {
-        for (long long i = tid; i < n_elem; i += 32 * kDecWarps) frame[i] = 0;
+    if (W > 1) {  // blocks that fail raise the status below
+        if (tid == 0 && status) status[c] = st;
+        __syncthreads();
+    } else if (lane == 0 && status) {
+        status[c] = st;
+    }
+    if (st != kStOk) {  // the same in every warp
+        for (long long i = tid; i < n_elem; i += 32 * W) frame[i] = 0;
         return;
     }
-    uint8_t* out_buf = wbuf + (size_t)warp * kBlockBytes;
-    for (int i = warp; i < n_blocks; i += kDecWarps) {
+    const bool vec = (n_elem & 7) == 0 && ((uintptr_t)out & 15u) == 0;
+    const bool wide = (n_elem & 15) == 0 && ((uintptr_t)out & 31u) == 0;
+    if (warp == 0) {  // raw leftover elements
+        const uint8_t* raw = ch + pos;
+        for (long long j = n8 + lane; j < n_elem; j += 32) {
+            const long long b = (j - n8) * 2;
+            frame[j] = (uint16_t)(raw[b] | (raw[b + 1] << 8));
+        }
+    }
+    pos = 12;
+    for (int i = 0; i < n_blocks; ++i) {
+        const int csz = (int)be32(ch + pos);
+        const uint8_t* in = ch + pos + 4;
+        pos += 4 + csz;
+        if (W > 1 && i % W != warp) continue;
         const long long e0 = (long long)i * kBlockElems;
         const int cnt = (int)min((long long)kBlockElems, n8 - e0);
-        const bool good = lz4_block_warp(ch + sh.start[i], sh.size[i], out_buf, 2 * cnt, lane);
+        const bool good = lz4_block_warp(in, csz, planes, 2 * cnt, lane);
         if (good) {
-            unshuffle_store(out_buf, cnt, frame + e0, vec, lane);
+            unshuffle_store(planes, cnt, frame + e0, vec, wide, lane);
         } else {
             for (int j = lane; j < cnt; j += 32) frame[e0 + j] = 0;
             if (lane == 0 && status) atomicMax(status + c, kStLz4);
         }
         __syncwarp();
-    }
-    if (warp == 0) {  // raw leftover elements
-        const uint8_t* raw = ch + sh.tail_at;
-        for (long long j = n8 + lane; j < n_elem; j += 32) {
-            const long long b = (j - n8) * 2;
-            frame[j] = (uint16_t)(raw[b] | (raw[b + 1] << 8));
-        }
     }
 }
 
@@ -237,17 +343,12 @@ __global__ void __launch_bounds__(32 * kDecWarps) k_decode_bslz4_u16(
 // Scratch layout: per (chunk, block) a slot of kEncSlot bytes holding the
 // big-endian compressed size followed by the LZ4 block.
 constexpr int kEncSlot = (4 + kLz4Bound + 15) & ~15;
-constexpr int kEncWarps = 4;
-// planes | hash table; the warps of a CTA share nothing
+// one warp per CTA: a block of zeros leaves its 16 KB to the next one at once
+// (with four, the blocks of one frame kept the slowest one's time: 645 us
+// at 4096 frames in the kernel)
+constexpr int kEncWarps = 1;
+// planes | hash table
 constexpr int kEncWarpBytes = kBlockBytes + 2 * kEncHash;
-
-// Four bytes at any byte position of a 4-aligned shared buffer. The second
-// word of an aligned position is read (it may be the first word of the hash
-// table) and shifted out.
-__device__ __forceinline__ uint32_t rd32(const uint8_t* base, int pos) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(base) + (pos >> 2);
-    return __funnelshift_r(w[0], w[1], 8 * (pos & 3));
-}
 
 // LZ4 length extension: x / 255 bytes of 255, then the rest. Returns the bytes written.
 __device__ __forceinline__ int put_length(uint8_t* o, int x, int lane) {
@@ -473,12 +574,17 @@ extern "C" int qssb_decode_bslz4_u16(const uint8_t* compressed, int64_t compress
     int rc = check_chunk_bytes(chunk_bytes, "qssb_decode_bslz4_u16: chunk_bytes must be even, "
                                             "at most 4 MB");
     if (rc) return rc;
-    const size_t smem = (size_t)kDecWarps * kBlockBytes;
-    CUDA_TRY(cudaFuncSetAttribute(k_decode_bslz4_u16, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)smem));
-    { k_decode_bslz4_u16<<<n_chunks, 32 * kDecWarps, smem, (cudaStream_t)stream>>>(
-        compressed, compressed_bytes, reinterpret_cast<const long long*>(chunk_offsets), n_chunks,
-        chunk_bytes, out, status); note_launch(); }
+    auto launch = [&](auto kern, int warps) {
+        kern<<<n_chunks, 32 * warps, 0, (cudaStream_t)stream>>>(
+            compressed, compressed_bytes, reinterpret_cast<const long long*>(chunk_offsets), n_chunks,
+            chunk_bytes, out, status);
+        note_launch();
+    };
+    // 27 warps of 8 KB fit an SM; fewer chunks than half of that take four warps each
+    if (n_chunks >= 13 * device_sm_count())
+        launch(k_decode_bslz4_u16<1>, 1);
+    else
+        launch(k_decode_bslz4_u16<kDecWarps>, kDecWarps);
     CUDA_TRY(cudaGetLastError());
     return QSSB_OK;
 }
