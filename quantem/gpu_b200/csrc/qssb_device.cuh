@@ -839,6 +839,107 @@ __device__ __forceinline__ T chi_full_poly(T dx, T dy, const FullChiT<T, T2>& f)
     return r2 * (f.c0[0] + r2 * (f.c0[1] + r2 * f.c0[2])) + re;
 }
 
+// The same chi split into its parts even and odd in u, both at the two
+// displacements of a pair in packed float32: lanes (x, y) = (q - k, q + k).
+// chi(u) = E(u) + O(u) and chi(-u) = E(u) - O(u), so one evaluation serves the
+// scan frequencies q and -q. The z^m of one parity step by z^2:
+//   E = r2 (K10 + r2 (K30 + r2 K50)) + Re z^2 (w_2 + z^2 (w_4 + z^2 w_6)),
+//   O = Re z (w_1 + z^2 (w_3 + z^2 w_5)),
+// w_m in r2 without the coefficients that no term has. `k`: the packed
+// coefficients of pack_full_chi, each twice (a packed operand of both lanes).
+constexpr int kFullPacked = 25;
+
+__device__ __forceinline__ void pack_full_chi(const FullChi& f, float2* k) {
+    const float v[kFullPacked] = {
+        f.c0[0],   f.c0[1],   f.c0[2],                                   // K10 K30 K50
+        f.w[1][0].x, f.w[1][0].y, f.w[1][1].x, f.w[1][1].y, f.w[1][2].x, f.w[1][2].y,  // w_2
+        f.w[3][0].x, f.w[3][0].y, f.w[3][1].x, f.w[3][1].y,              // w_4
+        f.w[5][0].x, f.w[5][0].y,                                        // w_6
+        f.w[0][1].x, f.w[0][1].y, f.w[0][2].x, f.w[0][2].y,              // w_1 = r2 (.. + r2 ..)
+        f.w[2][0].x, f.w[2][0].y, f.w[2][1].x, f.w[2][1].y,              // w_3
+        f.w[4][0].x, f.w[4][0].y};                                       // w_5
+#pragma unroll
+    for (int i = 0; i < kFullPacked; ++i) k[i] = make_float2(v[i], v[i]);
+}
+
+__device__ __forceinline__ void chi_full_pair(float2 x, float2 y, float2 r2, const float2* k,
+                                              float2& even, float2& odd) {
+    auto mul = [](float2 a, float2 b) { return __fmul2_rn(a, b); };
+    auto fma2 = [](float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); };
+    auto neg = [](float2 a) { return make_float2(-a.x, -a.y); };
+    const float2 xy = mul(x, y);
+    const float2 zr = fma2(x, x, neg(mul(y, y)));  // z^2
+    const float2 zi = __fadd2_rn(xy, xy);
+    // (sr + i si) z^2 + (wr + i wi)
+    auto step = [&](float2& sr, float2& si, float2 wr, float2 wi) {
+        const float2 tr = fma2(sr, zr, fma2(neg(si), zi, wr));
+        si = fma2(sr, zi, fma2(si, zr, wi));
+        sr = tr;
+    };
+    float2 sr = k[13], si = k[14];
+    step(sr, si, fma2(r2, k[11], k[9]), fma2(r2, k[12], k[10]));
+    step(sr, si, fma2(r2, fma2(r2, k[7], k[5]), k[3]), fma2(r2, fma2(r2, k[8], k[6]), k[4]));
+    const float2 c0 = fma2(r2, fma2(r2, k[2], k[1]), k[0]);
+    even = fma2(r2, c0, fma2(sr, zr, neg(mul(si, zi))));
+    sr = k[23], si = k[24];
+    step(sr, si, fma2(r2, k[21], k[19]), fma2(r2, k[22], k[20]));
+    step(sr, si, mul(r2, fma2(r2, k[17], k[15])), mul(r2, fma2(r2, k[18], k[16])));
+    odd = fma2(sr, x, neg(mul(si, y)));
+}
+
+// G conj(Gamma_hat) of Gamma = pm conj(pk) - conj(pp) pk (corrected_from_apertures).
+__device__ __forceinline__ float2 corrected_from_probes(float2 pm, float2 pp, float2 pk, float2 g) {
+    const float t1r = fmaf(pm.x, pk.x, pm.y * pk.y);
+    const float t1i = fmaf(pm.y, pk.x, -pm.x * pk.y);
+    const float t2r = fmaf(pp.x, pk.x, pp.y * pk.y);
+    const float t2i = fmaf(pp.x, pk.y, -pp.y * pk.x);
+    float gr = t1r - t2r;
+    float gi = t1i - t2i;
+    const float m2 = fmaf(gr, gr, gi * gi);
+    const float inv = m2 > 1e-16f ? rsqrtf(m2) : 1e8f;
+    gr *= inv;
+    gi *= inv;
+    return make_float2(fmaf(g.x, gr, g.y * gi), fmaf(g.y, gr, -g.x * gi));
+}
+
+// C(q) and C(-q) of one BF pixel with the 14-term chi. The apertures are even,
+// so both take the pair (A(q - k), A(q + k)), and G(-q) = conj G(q).
+__device__ __forceinline__ void corrected_full_pair(float qx, float qy, int r, int c, float kx,
+                                                    float ky, float kx_lo, float ky_lo, float2 pk,
+                                                    float2 g, const Probe& p, const float2* k,
+                                                    float2& v, float2& v_neg) {
+    const float2 x = make_float2(qx - kx, qx + kx);
+    const float2 y = make_float2(qy - ky, qy + ky);
+    const float2 r2 = __ffma2_rn(x, x, __fmul2_rn(y, y));
+    float am = soft_aperture(x.x, y.x, r2.x, p);
+    float ap = soft_aperture(x.y, y.y, r2.y, p);
+    if (fabsf(am - ap) < kApertureTie && (in_edge_band(r2.x, p) || in_edge_band(r2.y, p))) {
+        const double qx64 = fftfreq_d(r, p.n_r, p.qval_r);
+        const double qy64 = fftfreq_d(c, p.n_c, p.qval_c);
+        const double kx64 = (double)kx + (double)kx_lo;
+        const double ky64 = (double)ky + (double)ky_lo;
+        am = soft_aperture_fp64(qx64 - kx64, qy64 - ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
+        ap = soft_aperture_fp64(qx64 + kx64, qy64 + ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
+    }
+    v = v_neg = make_float2(0.0f, 0.0f);
+    if (am == 0.0f && ap == 0.0f) return;  // Gamma == 0
+    float2 even, odd;
+    chi_full_pair(x, y, r2, k, even, odd);
+    const float2 chi = __fadd2_rn(even, odd);
+    const float2 chi_neg = __fadd2_rn(even, make_float2(-odd.x, -odd.y));
+    float s, co;
+    sincosf(chi.x, &s, &co);
+    const float2 pm = make_float2(am * co, -am * s);  // P(q - k)
+    sincosf(chi.y, &s, &co);
+    const float2 pp = make_float2(ap * co, -ap * s);  // P(q + k)
+    v = corrected_from_probes(pm, pp, pk, g);
+    sincosf(chi_neg.y, &s, &co);
+    const float2 qm = make_float2(ap * co, -ap * s);  // P(-q - k)
+    sincosf(chi_neg.x, &s, &co);
+    const float2 qp = make_float2(am * co, -am * s);  // P(-q + k)
+    v_neg = corrected_from_probes(qm, qp, pk, cconj(g));
+}
+
 // C = G conj(Gamma_hat) (as `corrected`) with the 14-term chi at q -+ k.
 // CHI64: chi from FP64 q and k (k = kx + kx_lo), reduced to [-pi, pi] in FP64.
 template <bool CHI64>

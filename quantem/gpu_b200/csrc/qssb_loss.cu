@@ -2182,6 +2182,163 @@ __global__ void __launch_bounds__(kLossThreads, 1) k_loss_full(
     for (int i = tid; i < N * N; i += kLossThreads) pq[i] = sq[i];
 }
 
+// The 128 x 128 scan in float32 chi. A CTA per (BF chunk, candidate), one per
+// SM (the 128 x 129 plane and the groups' transposes: 211 KB). Per BF pixel:
+//  A) C on the half set of elem_rc128; an evaluation at (r, c), 1 <= r <= 63,
+//     c != 64, also gives C(-r, -c) (corrected_full_pair: chi's even and odd
+//     parts and the aperture pair are shared, both displacements in packed
+//     float32); the next element's G is loaded one ahead;
+//  B) row and C) column inverse FFTs by groups of 8 lanes (fft128_g8), phi per
+//     pixel in registers, phi^2 per thread in FP64, as k_loss_pair128.
+// Issue-bound: 8383 evaluations and 256 line FFTs per pixel. The form with
+// every frequency evaluated on its own and the shared-memory Stockham FFT
+// (k_loss_full, which other sizes and the FP64 chi keep) took 6.2 ms for 8
+// candidates of 1789 BF pixels; this one 3.5.
+struct Full128Smem {
+    static constexpr int pk_entries = 256;  // P(k_b) of the next BF pixels
+    static constexpr size_t s = sizeof(float2) * 128 * kL128P;
+    static constexpr size_t t = sizeof(float2) * 64 * kG8Scratch;
+    static constexpr size_t tw = sizeof(float2) * 128;
+    static constexpr size_t pk = sizeof(float2) * pk_entries;
+    static constexpr size_t bytes = s + t + tw + pk;
+};
+
+__global__ void __launch_bounds__(512, 1) k_loss_full128(
+    const float2* __restrict__ g, int n_bf, const float* __restrict__ geom,
+    const float* __restrict__ q_row, const float* __restrict__ q_col,
+    const qssb_full_aberrations_t* __restrict__ cands, qssb_calibration_t cal, int bf_per_chunk,
+    int n_chunks, float* __restrict__ part, double* __restrict__ part_sq) {
+    constexpr int N = 128;
+    constexpr int H = N / 2 + 1;
+    constexpr int P = kL128P;
+    extern __shared__ float4 smem4[];
+    char* base = reinterpret_cast<char*>(smem4);
+    float2* S = reinterpret_cast<float2*>(base);
+    float2* T = reinterpret_cast<float2*>(base + Full128Smem::s);
+    float2* tw = reinterpret_cast<float2*>(base + Full128Smem::s + Full128Smem::t);
+    float2* pks = tw + N;
+    __shared__ FullConsts sh;
+    __shared__ float2 packed[kFullPacked];
+    __shared__ double s_red[16];
+    const int tid = threadIdx.x;
+    const int lane = tid & 31;
+    const int warp = tid >> 5;
+    const int grp = lane >> 3;
+    const int s = lane & 7;
+    float2* Tg = T + (warp * 4 + grp) * kG8Scratch;
+    const int chunk = blockIdx.x;
+    const int cand = blockIdx.y;
+    if (tid == 0) {
+        load_full_consts(sh, cands, cand, cal);
+        pack_full_chi(sh.f, packed);
+    }
+    fill_twiddles<N>(tw, tid, 512);
+    __syncthreads();
+    const Probe& p = sh.p;
+    // the line (row or column) of this group within a round of 64
+    const int line = (warp & 7) + 8 * grp + 32 * (warp >> 3);
+    float acc[2][16];
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int t = 0; t < 16; ++t) acc[r][t] = 0.0f;
+    double sq = 0.0;
+    const int b0 = chunk * bf_per_chunk;
+    int nb = n_bf - b0;
+    if (nb > bf_per_chunk) nb = bf_per_chunk;
+    const float2 dc = make_float2((float)cal.dc_re, (float)cal.dc_im);
+    for (int i = 0; i < nb; ++i) {
+        const int b = b0 + i;
+        if (i % Full128Smem::pk_entries == 0) {
+            if (tid < Full128Smem::pk_entries && i + tid < nb) {
+                const int bt = b + tid;
+                pks[tid] = probe_full_at_bf(
+                    (double)__ldg(geom + bt) + (double)__ldg(geom + 6 * n_bf + bt),
+                    (double)__ldg(geom + n_bf + bt) + (double)__ldg(geom + 7 * n_bf + bt),
+                    __ldg(geom + 5 * n_bf + bt), sh.d);
+            }
+            __syncthreads();
+        }
+        const float kx = __ldg(geom + b);
+        const float ky = __ldg(geom + n_bf + b);
+        const float kx_lo = __ldg(geom + 6 * n_bf + b);
+        const float ky_lo = __ldg(geom + 7 * n_bf + b);
+        const float2 pk = pks[i % Full128Smem::pk_entries];
+        const float2* gb = g + (size_t)b * N * H;
+        auto gofs = [](int r, int c) {
+            return c <= N / 2 ? r * H + c : ((N - r) & (N - 1)) * H + (N - c);
+        };
+        float2 g_next;
+        {
+            int r, c;
+            elem_rc128(tid, r, c);  // tid < 512 < kNE128
+            g_next = __ldg(gb + gofs(r, c));
+        }
+        for (int e = tid; e < kNE128; e += 512) {
+            int r, c;
+            elem_rc128(e, r, c);
+            float2 gv = g_next;
+            if (e + 512 < kNE128) {
+                int rn, cn;
+                elem_rc128(e + 512, rn, cn);
+                g_next = __ldg(gb + gofs(rn, cn));
+            }
+            if (c > N / 2) gv.y = -gv.y;
+            float2 v, v_neg;
+            corrected_full_pair(__ldg(q_row + r), __ldg(q_col + c), r, c, kx, ky, kx_lo, ky_lo, pk,
+                                gv, p, packed, v, v_neg);
+            S[r * P + c] = e == 0 ? dc : v;
+            // the Nyquist row and column have no -q on the grid
+            if (r >= 1 && r < N / 2 && c != N / 2) S[(N - r) * P + ((N - c) & (N - 1))] = v_neg;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int round = 0; round < 2; ++round) {
+            float2* rowp = S + (line + 64 * round) * P;
+            float2 v[16];
+#pragma unroll
+            for (int n1 = 0; n1 < 16; ++n1) v[n1] = rowp[s + 8 * n1];
+            fft128_g8<+1>(v, Tg, s, tw);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) rowp[fft128_g8_index(s, t)] = v[t];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int round = 0; round < 2; ++round) {
+            const int x = line + 64 * round;
+            float2 v[16];
+#pragma unroll
+            for (int n1 = 0; n1 < 16; ++n1) v[n1] = S[(s + 8 * n1) * P + x];
+            fft128_g8<+1>(v, Tg, s, tw);
+#pragma unroll
+            for (int t = 0; t < 16; ++t) {
+                const float ph = phase_atan2(v[t].y, v[t].x);
+                sq = fma((double)ph, (double)ph, sq);
+                acc[round][t] += ph;
+            }
+        }
+        __syncthreads();
+    }
+    // row-major partial sum planes, as k_loss_pair128's
+    float* ps = part + (size_t)(cand * n_chunks + chunk) * N * N;
+#pragma unroll
+    for (int round = 0; round < 2; ++round) {
+        const int x = line + 64 * round;
+#pragma unroll
+        for (int t = 0; t < 16; ++t) ps[fft128_g8_index(s, t) * N + x] = acc[round][t];
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+    if (lane == 0) s_red[warp] = sq;
+    __syncthreads();
+    if (tid == 0) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < 16; ++w) t += s_red[w];
+        part_sq[cand * n_chunks + chunk] = t;
+    }
+}
+
 template <int N, bool CHI64>
 static int launch_loss_full(const float* g_half, const float* geom, const float* q_row,
                             const float* q_col, const qssb_calibration_t& cal,
@@ -2195,6 +2352,22 @@ static int launch_loss_full(const float* g_half, const float* geom, const float*
             g_half, geom, q_row, q_col, cal, cands, n_cand, pl, nullptr, part,
             ws + pl.part_bytes + pl.var_bytes, s);
         if (rc) return rc;
+    } else if constexpr (N == 128 && !CHI64) {
+        // sum planes (one per chunk), then one double per chunk
+        double* part_sq = reinterpret_cast<double*>(part + (size_t)n_cand * pl.n_chunks * N * N);
+        CUDA_TRY(cudaFuncSetAttribute(k_loss_full128, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)Full128Smem::bytes));
+        { k_loss_full128<<<dim3(pl.n_chunks, n_cand), 512, Full128Smem::bytes, s>>>(
+            reinterpret_cast<const float2*>(g_half), cal.n_bf, geom, q_row, q_col, cands, cal,
+            pl.bf_per_chunk, pl.n_chunks, part, part_sq); note_launch(); }
+        CUDA_TRY(cudaGetLastError());
+        { k_loss_reduce_sum<N><<<dim3(N * N / kReducePix, n_cand), kReducePix * kReduceSlices, 0, s>>>(
+            part, pl.n_chunks, cal.n_bf, var, mean_phase); note_launch(); }
+        CUDA_TRY(cudaGetLastError());
+        { k_loss_final_sq<<<n_cand, 256, 0, s>>>(var, N * N / kReducePix, part_sq, pl.n_chunks,
+                                               cal.n_bf, N * N, losses); note_launch(); }
+        CUDA_TRY(cudaGetLastError());
+        return QSSB_OK;
     } else {
         const size_t smem = LossSmem<N>::bytes + sizeof(float) * N * N;
         CUDA_TRY(cudaFuncSetAttribute(k_loss_full<N, CHI64>,
