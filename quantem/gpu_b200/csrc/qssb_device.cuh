@@ -397,6 +397,8 @@ struct Probe {
     // chi(u) = u^T M u for the quadratic (C10, C12) part; M symmetric
     float mxx, mxy, myy;
     double mxx_d, mxy_d, myy_d;
+    float mxy2;       // 2 mxy
+    float k30;        // (pi / lambda) lambda^4 C30 / 2: the coefficient of r2^2
     bool quadratic;   // C30 == 0: the factorised overlap applies
     double factor_d;  // FP64 copies for QSSB_FLAG_CHI_FP64
     double C10_d;
@@ -421,6 +423,14 @@ __device__ __forceinline__ float soft_aperture(float dx, float dy, float r2, con
     const float denom = sqrtf(num2) * inv_r;
     const float edge = denom > 1e-15f ? (p.semiangle - alpha) / denom + 0.5f : 1.0f;
     return fminf(fmaxf(edge, 0.0f), 1.0f);
+}
+
+// The same for isotropic sampling, where denom is the sampling itself: one
+// IEEE square root, two roundings fewer than soft_aperture and no branch.
+__device__ __forceinline__ float soft_aperture_iso(float r2, const Probe& p) {
+    const float edge = fmaf(fmaf(-sqrtf(r2), p.wavelength, p.semiangle), p.inv_ang, 0.5f);
+    const float a = r2 >= p.outer2 ? 0.0f : __saturatef(edge);
+    return r2 <= p.inner2 ? 1.0f : a;  // inner2 >= 0, so r2 == 0 gives 1
 }
 
 // The same aperture without branches and with reciprocal square roots only
@@ -571,6 +581,49 @@ __device__ __forceinline__ float2 corrected_from_apertures(const Disp& dm, const
     return make_float2(fmaf(g.x, gr, g.y * gi), fmaf(g.y, gr, -g.x * gi));
 }
 
+// chi (C10, C12, C30) at both displacements of a pair in packed float32, lanes
+// (x, y) = (q - k, q + k), as the polynomial x^T M x + K30 r2^2: chi_value
+// without cos 2phi and sin 2phi, so without their division by r2.
+__device__ __forceinline__ float2 chi_pair(float2 x, float2 y, const Probe& p) {
+    auto both = [](float v) { return make_float2(v, v); };
+    const float2 x2 = __fmul2_rn(x, x);
+    const float2 y2 = __fmul2_rn(y, y);
+    const float2 r2 = __fadd2_rn(x2, y2);
+    const float2 q = __ffma2_rn(both(p.mxy2), __fmul2_rn(x, y), __fmul2_rn(both(p.myy), y2));
+    return __ffma2_rn(__fmul2_rn(both(p.k30), r2), r2, __ffma2_rn(both(p.mxx), x2, q));
+}
+
+// G conj(Gamma_hat) of Gamma = pm conj(pk) - conj(pp) pk (corrected_from_apertures).
+// REFINE: the scale 1 / |Gamma| by rsqrtf and a Newton step, without which every
+// corrected value carries rsqrtf's rounding.
+template <bool REFINE = false>
+__device__ __forceinline__ float2 corrected_from_probes(float2 pm, float2 pp, float2 pk, float2 g) {
+    const float t1r = fmaf(pm.x, pk.x, pm.y * pk.y);
+    const float t1i = fmaf(pm.y, pk.x, -pm.x * pk.y);
+    const float t2r = fmaf(pp.x, pk.x, pp.y * pk.y);
+    const float t2i = fmaf(pp.x, pk.y, -pp.y * pk.x);
+    float gr = t1r - t2r;
+    float gi = t1i - t2i;
+    const float m2 = fmaf(gr, gr, gi * gi);
+    const float y = rsqrtf(m2);
+    const float inv = m2 > 1e-16f ? (REFINE ? fmaf(0.5f * y, fmaf(-m2 * y, y, 1.0f), y) : y) : 1e8f;
+    gr *= inv;
+    gi *= inv;
+    return make_float2(fmaf(g.x, gr, g.y * gi), fmaf(g.y, gr, -g.x * gi));
+}
+
+// corrected_from_apertures in float32 chi, from the aperture pair a =
+// (A(q - k), A(q + k)) (evaluated, or of the per-geometry table).
+__device__ __forceinline__ float2 corrected_from_table(float2 a, float qx, float qy, float kx,
+                                                       float ky, float2 pk, float2 g, const Probe& p) {
+    const float2 chi = chi_pair(make_float2(qx - kx, qx + kx), make_float2(qy - ky, qy + ky), p);
+    float sm, cm, sp, cp;
+    __sincosf(chi.x, &sm, &cm);
+    __sincosf(chi.y, &sp, &cp);
+    return corrected_from_probes(make_float2(a.x * cm, -a.x * sm), make_float2(a.y * cp, -a.y * sp),
+                                 pk, g);
+}
+
 // C = G conj(Gamma_hat), Gamma = P(q-k) conj(P(k)) - conj(P(q+k)) P(k),
 // Gamma_hat = Gamma * (|Gamma|^2 > 1e-16 ? 1/|Gamma| : 1e8)
 // (gamma_mul_pk_onthefly, common.py:173-236). (r, c) index the scan
@@ -591,7 +644,8 @@ __device__ __forceinline__ float2 corrected(float qx, float qy, int r, int c, fl
         am = soft_aperture_fp64(qx64 - kx64, qy64 - ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
         ap = soft_aperture_fp64(qx64 + kx64, qy64 + ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
     }
-    return corrected_from_apertures<CHI64>(dm, dp, am, ap, pk, g, p);
+    if constexpr (CHI64) return corrected_from_apertures<CHI64>(dm, dp, am, ap, pk, g, p);
+    return corrected_from_table(make_float2(am, ap), qx, qy, kx, ky, pk, g, p);
 }
 
 // Probe constants of one candidate from the calibration (FP64 trig of phi12).
@@ -640,6 +694,8 @@ __host__ __device__ inline Probe make_probe_common(const qssb_calibration_t& cal
     p.mxx = (float)p.mxx_d;
     p.mxy = (float)p.mxy_d;
     p.myy = (float)p.myy_d;
+    p.mxy2 = (float)(2.0 * p.mxy_d);
+    p.k30 = (float)(0.5 * fl2 * cal.wavelength_A * cal.wavelength_A * (double)C30);
     p.quadratic = (C30 == 0.0f);
     return p;
 }
@@ -887,21 +943,6 @@ __device__ __forceinline__ void chi_full_pair(float2 x, float2 y, float2 r2, con
     odd = fma2(sr, x, neg(mul(si, y)));
 }
 
-// G conj(Gamma_hat) of Gamma = pm conj(pk) - conj(pp) pk (corrected_from_apertures).
-__device__ __forceinline__ float2 corrected_from_probes(float2 pm, float2 pp, float2 pk, float2 g) {
-    const float t1r = fmaf(pm.x, pk.x, pm.y * pk.y);
-    const float t1i = fmaf(pm.y, pk.x, -pm.x * pk.y);
-    const float t2r = fmaf(pp.x, pk.x, pp.y * pk.y);
-    const float t2i = fmaf(pp.x, pk.y, -pp.y * pk.x);
-    float gr = t1r - t2r;
-    float gi = t1i - t2i;
-    const float m2 = fmaf(gr, gr, gi * gi);
-    const float inv = m2 > 1e-16f ? rsqrtf(m2) : 1e8f;
-    gr *= inv;
-    gi *= inv;
-    return make_float2(fmaf(g.x, gr, g.y * gi), fmaf(g.y, gr, -g.x * gi));
-}
-
 // C(q) and C(-q) of one BF pixel with the 14-term chi. The apertures are even,
 // so both take the pair (A(q - k), A(q + k)), and G(-q) = conj G(q).
 __device__ __forceinline__ void corrected_full_pair(float qx, float qy, int r, int c, float kx,
@@ -911,8 +952,14 @@ __device__ __forceinline__ void corrected_full_pair(float qx, float qy, int r, i
     const float2 x = make_float2(qx - kx, qx + kx);
     const float2 y = make_float2(qy - ky, qy + ky);
     const float2 r2 = __ffma2_rn(x, x, __fmul2_rn(y, y));
-    float am = soft_aperture(x.x, y.x, r2.x, p);
-    float ap = soft_aperture(x.y, y.y, r2.y, p);
+    float am, ap;
+    if (p.iso) {  // denom is d_row in every direction
+        am = soft_aperture_iso(r2.x, p);
+        ap = soft_aperture_iso(r2.y, p);
+    } else {
+        am = soft_aperture(x.x, y.x, r2.x, p);
+        ap = soft_aperture(x.y, y.y, r2.y, p);
+    }
     if (fabsf(am - ap) < kApertureTie && (in_edge_band(r2.x, p) || in_edge_band(r2.y, p))) {
         const double qx64 = fftfreq_d(r, p.n_r, p.qval_r);
         const double qy64 = fftfreq_d(c, p.n_c, p.qval_c);
@@ -932,12 +979,12 @@ __device__ __forceinline__ void corrected_full_pair(float qx, float qy, int r, i
     const float2 pm = make_float2(am * co, -am * s);  // P(q - k)
     sincosf(chi.y, &s, &co);
     const float2 pp = make_float2(ap * co, -ap * s);  // P(q + k)
-    v = corrected_from_probes(pm, pp, pk, g);
+    v = corrected_from_probes<true>(pm, pp, pk, g);
     sincosf(chi_neg.y, &s, &co);
     const float2 qm = make_float2(ap * co, -ap * s);  // P(-q - k)
     sincosf(chi_neg.x, &s, &co);
     const float2 qp = make_float2(am * co, -am * s);  // P(-q + k)
-    v_neg = corrected_from_probes(qm, qp, pk, cconj(g));
+    v_neg = corrected_from_probes<true>(qm, qp, pk, cconj(g));
 }
 
 // C = G conj(Gamma_hat) (as `corrected`) with the 14-term chi at q -+ k.

@@ -581,11 +581,18 @@ __device__ __forceinline__ float2 corrected_table_direct(float2 a, float qx, flo
                                                          const Probe& p) {
     const float m = ak * a.x;
     const float l = ak * a.y;
-    const Disp dm = displacement(qx - kx, qy - ky, p);
-    const Disp dp = displacement(qx + kx, qy + ky, p);
+    float2 chi;  // at q - k and q + k
+    if constexpr (CHI64) {
+        const Disp dm = displacement(qx - kx, qy - ky, p);
+        const Disp dp = displacement(qx + kx, qy + ky, p);
+        chi = make_float2(chi_value<CHI64>(dm.alpha2, dm.cos2, dm.sin2, p),
+                          chi_value<CHI64>(dp.alpha2, dp.cos2, dp.sin2, p));
+    } else {
+        chi = chi_pair(make_float2(qx - kx, qx + kx), make_float2(qy - ky, qy + ky), p);
+    }
     float sm, cm, sp, cp;
-    __sincosf(chi_value<CHI64>(dm.alpha2, dm.cos2, dm.sin2, p), &sm, &cm);
-    __sincosf(chi_value<CHI64>(dp.alpha2, dp.cos2, dp.sin2, p), &sp, &cp);
+    __sincosf(chi.x, &sm, &cm);
+    __sincosf(chi.y, &sp, &cp);
     // t1 = m (cm - i sm)(ck + i sk), t2 = l (cp + i sp)(ck - i sk)
     const float t1r = m * fmaf(cm, ek.x, sm * ek.y);
     const float t1i = m * fmaf(cm, ek.y, -sm * ek.x);
@@ -1017,8 +1024,8 @@ __global__ void __launch_bounds__(256) k_loss_final_sq(const double* __restrict_
 
 // ---------------------------------------------- N >= 256: two passes
 // A 256^2 .. 1024^2 plane does not fit one CTA's shared memory. The BF pixels
-// are taken in chunks whose row-transformed planes stay in L2 (about 48 MB
-// for all candidates of the call):
+// are taken in chunks whose row-transformed planes stay in L2 (kStageBudget
+// for the candidates of a group):
 //   k_loss_rows: one warp per row of C_b (rows 0..N/2 on the +-q half set, all
 //     N rows for the 14-term chi): evaluate, inverse-FFT, store the row in the
 //     chunk's staging planes; the half-set path also stores
@@ -1031,7 +1038,12 @@ __global__ void __launch_bounds__(256) k_loss_final_sq(const double* __restrict_
 //     of its pixels in registers; at the end of the chunk it adds them to its
 //     own partial planes (column-major), so every element has one writer.
 constexpr int kL256 = 256;
-constexpr size_t kStageBudget = 32u << 20;
+// Staging of one chunk. Twice the chunk halves the launches and their ramps
+// (16 candidates with C30 at 256^2: 18.5 ms with 32 MB, 17.0 with 64) and
+// still stays in L2. The quadratic loss at 256^2 keeps 32 MB: the persistent
+// launch holds three such slots in L2 and has the launch sequence's chunks.
+constexpr size_t kStageBudget = 64u << 20;
+constexpr size_t kStageBudgetQueue = 32u << 20;
 // The persistent one-launch loss (k_loss_queue, QSSB_FLAG_PERSISTENT): 256^2,
 // half set, float32 chi, at most this many candidate groups (27 candidates each).
 constexpr int kQueueN = 256;
@@ -1054,6 +1066,10 @@ static bool loss_queue_requested(int n, int flags) {
 // CTAs per SM (80 registers) hide more latency than one 16-warp CTA at 128.
 __host__ __device__ constexpr int row_warps(int n) { return n >= 1024 ? 8 : (n == 256 ? 8 : 16); }
 __host__ __device__ constexpr int row_min_ctas(int n) { return n == 256 ? 3 : 1; }
+// The 14-term chi's CTA starts with FP64 work (its coefficients, P(k)), shared
+// by four rows a warp at 256^2 (2 candidates of 1789 BF pixels: 9.0 ms with one
+// row a warp, 6.9 with four); the half set measured the same either way.
+__host__ __device__ constexpr int rows_per_warp(int n, bool full) { return full && n == 256 ? 4 : 1; }
 __host__ __device__ constexpr int row_load_batch(int n) { return n == 256 ? 4 : 8; }
 __host__ __device__ constexpr int col_tile(int n) { return n >= 1024 ? 8 : 16; }
 
@@ -1065,7 +1081,9 @@ struct TwoPass {
     // CTA after its row 0, so the rows 0 .. N/2 - 1 fill whole CTAs (17 CTAs
     // of 8 warps would leave one CTA a single row)
     static constexpr bool fold_nyquist = !FULL && N == 256;
-    static constexpr int row_ctas = fold_nyquist ? N / 2 / rwarps : (rows + rwarps - 1) / rwarps;
+    static constexpr int row_block = rwarps * rows_per_warp(N, FULL);  // rows of one CTA
+    static constexpr int row_ctas =
+        fold_nyquist ? N / 2 / row_block : (rows + row_block - 1) / row_block;
     static constexpr int tile = col_tile(N);
     static constexpr int scratch = warp_fft_scratch<N>();
     // column line pitch: odd mod 16 (conflict-free strip loads), and room for
@@ -1100,7 +1118,8 @@ struct TwoPassPlan {
 // read-modify-write of its partial planes (a whole 64-candidate batch at once
 // leaves one pixel per chunk). Full waves beat equal groups: 27/27/10 takes
 // 1.14 ms per candidate at 256^2 against 1.24 for 22/22/20.
-static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chunks_req) {
+static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chunks_req,
+                                 size_t budget) {
     TwoPassPlan tp;
     const int strips = n / col_tile(n);
     // column-pass CTA slots of the B200 (148 SMs); groups of equal size
@@ -1110,8 +1129,23 @@ static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chu
     if (group > n_cand) group = n_cand;
     tp.group = group;
     const size_t per_bf = sizeof(float2) * (size_t)(full ? n : n / 2 + 1) * n;
-    long long c = (long long)(kStageBudget / (per_bf * (size_t)group));
+    long long c = (long long)(budget / (per_bf * (size_t)group));
     if (c < 1) c = 1;
+    if (full && n == 256) {
+        // the chunk, from the budget down to half of it, whose row pass fills its
+        // waves best (an item is 32 rows, so a last wave is a larger share)
+        const long long items = (long long)TwoPass<256, true>::row_ctas * group;
+        const long long rslots = 148LL * row_min_ctas(n);
+        double best = 0.0;
+        for (long long k = c, kmin = (c + 1) / 2; k >= kmin; --k) {
+            const long long waves = (items * k + rslots - 1) / rslots;
+            const double fill = (double)(items * k) / (double)(waves * rslots);
+            if (fill > best + 1e-9) {
+                best = fill;
+                c = k;
+            }
+        }
+    }
     if (c > n_bf) c = n_bf;
     tp.chunk_bf = (int)c;
     // whole waves of the column pass's CTA slots, not a last partial wave
@@ -1142,13 +1176,18 @@ __device__ __forceinline__ void loss_rows_item(
     __shared__ FullChi sf;
     __shared__ FullChi64 sd;
     __shared__ float2 s_phc[kSep ? N : 1];
-    __shared__ float2 s_phr[kSep ? RW : 1];
+    constexpr int RB = TP::row_block;
+    __shared__ float2 s_phr[kSep ? RB : 1];
+    // the Nyquist column of the CTA's rows: conj C(r, N/2) and C(-r, N/2)
+    __shared__ float2 s_ny[FULL ? 1 : RB];
+    __shared__ float2 s_partner[FULL ? 1 : RB];
+    static_assert(FULL || RB <= 32, "one warp evaluates the partners");
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
     const int b = b0 + bi;
     const int cand = cand0 + zc;
-    const int r0 = rowblock * RW;
+    const int r0 = rowblock * RB;
     {  // the candidate's probe, from k_two_pass_setup
         const auto* src = reinterpret_cast<const unsigned int*>(probes + cand);
         auto* dst = reinterpret_cast<unsigned int*>(&sp);
@@ -1172,7 +1211,7 @@ __device__ __forceinline__ void loss_rows_item(
                                 __ldg(geom + 4 * n_bf + b), __ldg(geom + 5 * n_bf + b), p);
     }
     if constexpr (kSep) {  // e^{i 2 q_col(c) v} for all columns, e^{i 2 q_row(r) u} for this CTA's rows
-        for (int i = tid; i < N + RW; i += 32 * RW) {
+        for (int i = tid; i < N + RB; i += 32 * RW) {
             float sn, cs;
             if (i < N) {
                 sincosf(2.0f * __ldg(q_col + i) * kq.v, &sn, &cs);
@@ -1211,7 +1250,9 @@ __device__ __forceinline__ void loss_rows_item(
         } else if constexpr (QUAD) {
             return corrected_quad<CHI64>(qx, qy, rr, c, eq, kq, gv, p);
         } else {
-            if (tab) {
+            if constexpr (!CHI64) {
+                if (tab) return corrected_from_table(ov, qx, qy, kq.kx, kq.ky, pk, gv, p);
+            } else if (tab) {
                 const Disp dm = displacement(qx - kq.kx, qy - kq.ky, p);
                 const Disp dp = displacement(qx + kq.kx, qy + kq.ky, p);
                 return corrected_from_apertures<CHI64>(dm, dp, ov.x, ov.y, pk, gv, p);
@@ -1241,21 +1282,8 @@ __device__ __forceinline__ void loss_rows_item(
                 const int t = t0 + u;
                 const int c = lane + 32 * t;
                 v[t] = (r == 0 && c == 0) ? dc : eval(r, c, qx, qy[u], gv[u], eq[u], e_row, ov[u]);
-                if (!FULL && t == N / 64 && lane == 0 && r >= 1 && r < N / 2) {  // c == N/2
-                    float2 e_neg = make_float2(1.0f, 0.0f);
-                    if constexpr (kSep) {
-                        float sn, cs;
-                        sincosf(2.0f * __ldg(q_row + N - r) * kq.u, &sn, &cs);
-                        e_neg = make_float2(cs, sn);
-                    }
-                    const float2 eqn = QUAD && !FULL ? __ldg(eqc + (N - r) * N + N / 2)
-                                                     : make_float2(1.0f, 0.0f);
-                    const float2 ovn =
-                        tab ? __ldg(ovb + (N / 2 + 1) * N + r) : make_float2(0.0f, 0.0f);
-                    const float2 partner = eval(N - r, N / 2, __ldg(q_row + N - r), qy[u],
-                                                load_g(N - r, N / 2), eqn, e_neg, ovn);
-                    delta[((size_t)zc * nb_chunk + bi) * (N / 2) + r] =
-                        cadd(cconj(v[t]), partner);
+                if constexpr (!FULL) {
+                    if (t == N / 64 && lane == 0 && r < N / 2) s_ny[r - r0] = cconj(v[t]);  // c == N/2
                 }
             }
         }
@@ -1264,12 +1292,39 @@ __device__ __forceinline__ void loss_rows_item(
 #pragma unroll
         for (int j = 0; j < RPL; ++j) out[warp_fft_index<N>(lane, j)] = v[j];
     };
-    const int r = r0 + warp;
-    if (r < TP::rows) row(r, kSep ? s_phr[warp] : make_float2(1.0f, 0.0f));
+    if constexpr (!FULL) {
+        // the partners C(-r, N/2) of the CTA's rows, one lane each
+        const int r = r0 + lane;
+        if (warp == RW - 1 && lane < RB && r >= 1 && r < N / 2) {
+            float2 e_neg = make_float2(1.0f, 0.0f);
+            if constexpr (kSep) {
+                float sn, cs;
+                sincosf(2.0f * __ldg(q_row + N - r) * kq.u, &sn, &cs);
+                e_neg = make_float2(cs, sn);
+            }
+            const float2 eqn =
+                QUAD ? __ldg(eqc + (N - r) * N + N / 2) : make_float2(1.0f, 0.0f);
+            const float2 ovn = tab ? __ldg(ovb + (N / 2 + 1) * N + r) : make_float2(0.0f, 0.0f);
+            s_partner[lane] = eval(N - r, N / 2, __ldg(q_row + N - r), __ldg(q_col + N / 2),
+                                   load_g(N - r, N / 2), eqn, e_neg, ovn);
+        }
+    }
+#pragma unroll 1
+    for (int j = 0; j < rows_per_warp(N, FULL); ++j) {
+        const int r = r0 + warp + RW * j;
+        if (r >= TP::rows) break;
+        row(r, kSep ? s_phr[r - r0] : make_float2(1.0f, 0.0f));
+        __syncwarp();  // the FFT scratch is reused
+    }
+    if constexpr (!FULL) {
+        __syncthreads();
+        const int r = r0 + tid;
+        if (tid < RB && r >= 1 && r < N / 2)
+            delta[((size_t)zc * nb_chunk + bi) * (N / 2) + r] = cadd(s_ny[tid], s_partner[tid]);
+    }
     if constexpr (TP::fold_nyquist) {
-        static_assert(TP::row_ctas * RW == N / 2, "whole CTAs of rows");
+        static_assert(TP::row_ctas * RB == N / 2, "whole CTAs of rows");
         if (rowblock == 0 && warp == 0) {
-            __syncwarp();  // the FFT scratch is reused by the Nyquist row
             float2 e_row = make_float2(1.0f, 0.0f);
             if constexpr (kSep) {
                 float sn, cs;
@@ -1578,14 +1633,16 @@ struct LossPlan {
 // Deterministic: about 296 CTAs in total (two per B200 SM), at least one BF
 // pixel each. N >= 256: the two-pass plan (n_chunks = its column interleave).
 static LossPlan plan_loss(int n, int n_bf, int n_cand, int chunks_req = 0, bool full = false,
-                          bool queue = false) {
+                          bool queue = false, bool quad = false) {
     LossPlan pl;
     pl.queue = false;
     pl.n_groups = 0;
     pl.n_phase_chunks = 0;
     pl.queue_bytes = 0;
     if (n >= kL256) {
-        const TwoPassPlan tp = plan_two_pass(n, full, n_bf, n_cand, chunks_req);
+        const bool small = n == kQueueN && !full && (queue || quad);
+        const TwoPassPlan tp = plan_two_pass(n, full, n_bf, n_cand, chunks_req,
+                                             small ? kStageBudgetQueue : kStageBudget);
         pl.chunk_bf = tp.chunk_bf;
         pl.n_chunks = tp.n_sub;
         pl.bf_per_chunk = 0;
@@ -1979,7 +2036,8 @@ static int launch_loss(const float* g_half, const float* geom, const float* q_ro
                        const qssb_aberrations_t* cands, int n_cand, int flags, char* ws,
                        float* losses, float* mean_phase, const float2* overlap, cudaStream_t s) {
     const LossPlan pl = plan_loss(N, cal.n_bf, n_cand, flag_chunks(flags), false,
-                                  loss_queue_requested(N, flags));
+                                  loss_queue_requested(N, flags),
+                                  (flags & QSSB_FLAG_QUADRATIC) != 0);
     float* part = reinterpret_cast<float*>(ws);
     double* var = reinterpret_cast<double*>(ws + pl.part_bytes);
     float2* eq = reinterpret_cast<float2*>(ws + pl.part_bytes + pl.var_bytes);
@@ -2193,7 +2251,7 @@ __global__ void __launch_bounds__(kLossThreads, 1) k_loss_full(
 // Issue-bound: 8383 evaluations and 256 line FFTs per pixel. The form with
 // every frequency evaluated on its own and the shared-memory Stockham FFT
 // (k_loss_full, which other sizes and the FP64 chi keep) took 6.2 ms for 8
-// candidates of 1789 BF pixels; this one 3.5.
+// candidates of 1789 BF pixels; this one 3.3.
 struct Full128Smem {
     static constexpr int pk_entries = 256;  // P(k_b) of the next BF pixels
     static constexpr size_t s = sizeof(float2) * 128 * kL128P;
@@ -2409,7 +2467,8 @@ extern "C" int qssb_loss_workspace_bytes(const qssb_calibration_t* cal, int32_t 
         return set_error(QSSB_ERR_UNSUPPORTED,
                          "qssb_loss_batch: scan size must be 64, 128, 256, 512 or 1024");
     const LossPlan pl =
-        plan_loss(n, cal->n_bf, n_cand, flag_chunks(flags), false, loss_queue_requested(n, flags));
+        plan_loss(n, cal->n_bf, n_cand, flag_chunks(flags), false, loss_queue_requested(n, flags),
+                  (flags & QSSB_FLAG_QUADRATIC) != 0);
     *bytes = loss_workspace(pl);
     return QSSB_OK;
 }
