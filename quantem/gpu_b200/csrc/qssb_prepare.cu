@@ -945,6 +945,26 @@ struct ScanLines {
     static constexpr size_t cols_smem = sizeof(float2) * ((size_t)kTile * P + N);
 };
 
+// Place of a spectrum's element in its shared line. The warp FFT leaves a lane
+// group's G = 32 / R elements N / G apart, on the same banks; shifting each
+// N / G elements by 16 / G spreads them (with none, the 4-way conflicts of
+// these stores at 256 held k_scan_rows at 93% of the L1 pipe).
+template <int N>
+__device__ __forceinline__ int line_place(int i) {
+    constexpr int G = 32 / (N / 32);
+    return G > 1 ? i + (i / (N / G)) * (16 / G) : i;
+}
+
+// Pitch of T staged columns: whole scratch and T neighbouring columns of a row
+// 16 / T apart mod 16, so that a half-warp's 16 / T rows x T columns meet no
+// bank twice. With both, the two passes over 1789 BF pixels at 256^2 take
+// 0.595 ms (0.642 with odd pitches and unshifted lines), over 1000 at 512^2
+// 0.99 (1.01).
+template <int N, int T>
+__host__ __device__ constexpr int strip_pitch() {
+    return (ScanLines<N>::kScratch + 15) / 16 * 16 + 16 / T;
+}
+
 // Rows: one warp per row pair, the line straight into registers
 // (v[t] = x[32 t + lane]), warp FFT, spectrum back to the warp's shared line
 // in natural order for the real-pair split.
@@ -976,13 +996,13 @@ __global__ void __launch_bounds__(32 * ScanLines<N>::kWarps) k_scan_rows(
     float2* x = scr + warp * L::kScratch;
     warp_fft<N, -1>(v, x, tw, lane);
 #pragma unroll
-    for (int j = 0; j < RPL; ++j) x[warp_fft_index<N>(lane, j)] = v[j];
+    for (int j = 0; j < RPL; ++j) x[line_place<N>(warp_fft_index<N>(lane, j))] = v[j];
     __syncwarp();
     float2* g0 = g_half + ((size_t)b * N + 2 * pair) * H;
     float2* g1 = g0 + H;
     for (int c = lane; c < H; c += 32) {
-        const float2 z = x[c];
-        const float2 m = x[(N - c) & (N - 1)];
+        const float2 z = x[line_place<N>(c)];
+        const float2 m = x[line_place<N>((N - c) & (N - 1))];
         g0[c] = make_float2(0.5f * (z.x + m.x), 0.5f * (z.y - m.y));
         g1[c] = make_float2(0.5f * (z.y + m.y), -0.5f * (z.x - m.x));
     }
@@ -1046,7 +1066,7 @@ __device__ __forceinline__ void scan_cp_async8(void* smem_dst, const void* gmem_
 template <int N, int T = ScanLines<N>::kTileP, int CTAS = ScanLines<N>::kCtasP>
 __global__ void __launch_bounds__(32 * T, CTAS) k_scan_cols_p(int n_bf, float2* __restrict__ g_half) {
     using L = ScanLines<N>;
-    constexpr int P = L::P;  // T: columns per strip, one warp each; CTAS: CTAs per SM
+    constexpr int P = strip_pitch<N, T>();  // T: columns per strip, one warp each; CTAS: CTAs per SM
     constexpr int NT = 32 * T;
     constexpr int H = L::H;
     constexpr int RPL = N / 32;
@@ -1089,14 +1109,14 @@ __global__ void __launch_bounds__(32 * T, CTAS) k_scan_cols_p(int n_bf, float2* 
             __syncwarp();
             warp_fft<N, -1>(v, line, tw, lane);
 #pragma unroll
-            for (int j = 0; j < RPL; ++j) line[warp_fft_index<N>(lane, j)] = v[j];
+            for (int j = 0; j < RPL; ++j) line[line_place<N>(warp_fft_index<N>(lane, j))] = v[j];
         }
         __syncthreads();
         float2* g = g_half + (size_t)b * N * H + c0;
         for (int e = tid; e < N * T; e += NT) {
             const int r = e / T;
             const int c = e - r * T;
-            if (c < nc) g[(size_t)r * H + c] = tile[c * P + r];
+            if (c < nc) g[(size_t)r * H + c] = tile[c * P + line_place<N>(r)];
         }
         buf ^= 1;
     }
@@ -1106,7 +1126,7 @@ __global__ void __launch_bounds__(32 * T, CTAS) k_scan_cols_p(int n_bf, float2* 
 template <int N, int T, int CTAS>
 static int launch_scan_cols_p(int n_bf, float2* g, cudaStream_t s) {
     using L = ScanLines<N>;
-    const size_t smem = sizeof(float2) * ((size_t)2 * T * L::P + N);
+    const size_t smem = sizeof(float2) * ((size_t)2 * T * strip_pitch<N, T>() + N);
     CUDA_TRY(cudaFuncSetAttribute(k_scan_cols_p<N, T, CTAS>,
                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const long long items = (long long)n_bf * ((L::H + T - 1) / T);
