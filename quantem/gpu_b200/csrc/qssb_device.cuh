@@ -944,8 +944,11 @@ __device__ __forceinline__ void chi_full_pair(float2 x, float2 y, float2 r2, con
 }
 
 // C(q) and C(-q) of one BF pixel with the 14-term chi. The apertures are even,
-// so both take the pair (A(q - k), A(q + k)), and G(-q) = conj G(q).
-__device__ __forceinline__ void corrected_full_pair(float qx, float qy, int r, int c, float kx,
+// so both take the pair (A(q - k), A(q + k)), and G(-q) = conj G(q). q_lo and
+// k_lo, the float32 residuals of q and k, enter chi's displacements: rounding q
+// and k moves chi by several times what its evaluation does.
+__device__ __forceinline__ void corrected_full_pair(float qx, float qy, float qx_lo, float qy_lo,
+                                                    int r, int c, float kx,
                                                     float ky, float kx_lo, float ky_lo, float2 pk,
                                                     float2 g, const Probe& p, const float2* k,
                                                     float2& v, float2& v_neg) {
@@ -970,8 +973,10 @@ __device__ __forceinline__ void corrected_full_pair(float qx, float qy, int r, i
     }
     v = v_neg = make_float2(0.0f, 0.0f);
     if (am == 0.0f && ap == 0.0f) return;  // Gamma == 0
+    const float2 xc = __fadd2_rn(x, make_float2(qx_lo - kx_lo, qx_lo + kx_lo));
+    const float2 yc = __fadd2_rn(y, make_float2(qy_lo - ky_lo, qy_lo + ky_lo));
     float2 even, odd;
-    chi_full_pair(x, y, r2, k, even, odd);
+    chi_full_pair(xc, yc, __ffma2_rn(xc, xc, __fmul2_rn(yc, yc)), k, even, odd);
     const float2 chi = __fadd2_rn(even, odd);
     const float2 chi_neg = __fadd2_rn(even, make_float2(-odd.x, -odd.y));
     float s, co;

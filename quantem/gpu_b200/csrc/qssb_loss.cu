@@ -2251,14 +2251,15 @@ __global__ void __launch_bounds__(kLossThreads, 1) k_loss_full(
 // Issue-bound: 8383 evaluations and 256 line FFTs per pixel. The form with
 // every frequency evaluated on its own and the shared-memory Stockham FFT
 // (k_loss_full, which other sizes and the FP64 chi keep) took 6.2 ms for 8
-// candidates of 1789 BF pixels; this one 3.3.
+// candidates of 1789 BF pixels; this one 2.8.
 struct Full128Smem {
     static constexpr int pk_entries = 256;  // P(k_b) of the next BF pixels
     static constexpr size_t s = sizeof(float2) * 128 * kL128P;
     static constexpr size_t t = sizeof(float2) * 64 * kG8Scratch;
     static constexpr size_t tw = sizeof(float2) * 128;
     static constexpr size_t pk = sizeof(float2) * pk_entries;
-    static constexpr size_t bytes = s + t + tw + pk;
+    static constexpr size_t q = sizeof(float2) * 256;  // (q, its residual) by row, by column
+    static constexpr size_t bytes = s + t + tw + pk + q;
 };
 
 __global__ void __launch_bounds__(512, 1) k_loss_full128(
@@ -2275,6 +2276,7 @@ __global__ void __launch_bounds__(512, 1) k_loss_full128(
     float2* T = reinterpret_cast<float2*>(base + Full128Smem::s);
     float2* tw = reinterpret_cast<float2*>(base + Full128Smem::s + Full128Smem::t);
     float2* pks = tw + N;
+    float2* qs = pks + Full128Smem::pk_entries;
     __shared__ FullConsts sh;
     __shared__ float2 packed[kFullPacked];
     __shared__ double s_red[16];
@@ -2293,6 +2295,12 @@ __global__ void __launch_bounds__(512, 1) k_loss_full128(
     fill_twiddles<N>(tw, tid, 512);
     __syncthreads();
     const Probe& p = sh.p;
+    if (tid < 256) {
+        const int j = tid & 127;
+        const float q = __ldg(tid < 128 ? q_row + j : q_col + j);
+        const double q64 = tid < 128 ? fftfreq_d(j, N, p.qval_r) : fftfreq_d(j, N, p.qval_c);
+        qs[tid] = make_float2(q, (float)(q64 - (double)q));
+    }
     // the line (row or column) of this group within a round of 64
     const int line = (warp & 7) + 8 * grp + 32 * (warp >> 3);
     float acc[2][16];
@@ -2343,8 +2351,9 @@ __global__ void __launch_bounds__(512, 1) k_loss_full128(
             }
             if (c > N / 2) gv.y = -gv.y;
             float2 v, v_neg;
-            corrected_full_pair(__ldg(q_row + r), __ldg(q_col + c), r, c, kx, ky, kx_lo, ky_lo, pk,
-                                gv, p, packed, v, v_neg);
+            const float2 qr = qs[r], qc = qs[N + c];
+            corrected_full_pair(qr.x, qc.x, qr.y, qc.y, r, c, kx, ky, kx_lo, ky_lo, pk, gv, p, packed,
+                                v, v_neg);
             S[r * P + c] = e == 0 ? dc : v;
             // the Nyquist row and column have no -q on the grid
             if (r >= 1 && r < N / 2 && c != N / 2) S[(N - r) * P + ((N - c) & (N - 1))] = v_neg;
