@@ -397,8 +397,6 @@ struct Probe {
     // chi(u) = u^T M u for the quadratic (C10, C12) part; M symmetric
     float mxx, mxy, myy;
     double mxx_d, mxy_d, myy_d;
-    float mxy2;       // 2 mxy
-    float k30;        // (pi / lambda) lambda^4 C30 / 2: the coefficient of r2^2
     bool quadratic;   // C30 == 0: the factorised overlap applies
     double factor_d;  // FP64 copies for QSSB_FLAG_CHI_FP64
     double C10_d;
@@ -581,18 +579,6 @@ __device__ __forceinline__ float2 corrected_from_apertures(const Disp& dm, const
     return make_float2(fmaf(g.x, gr, g.y * gi), fmaf(g.y, gr, -g.x * gi));
 }
 
-// chi (C10, C12, C30) at both displacements of a pair in packed float32, lanes
-// (x, y) = (q - k, q + k), as the polynomial x^T M x + K30 r2^2: chi_value
-// without cos 2phi and sin 2phi, so without their division by r2.
-__device__ __forceinline__ float2 chi_pair(float2 x, float2 y, const Probe& p) {
-    auto both = [](float v) { return make_float2(v, v); };
-    const float2 x2 = __fmul2_rn(x, x);
-    const float2 y2 = __fmul2_rn(y, y);
-    const float2 r2 = __fadd2_rn(x2, y2);
-    const float2 q = __ffma2_rn(both(p.mxy2), __fmul2_rn(x, y), __fmul2_rn(both(p.myy), y2));
-    return __ffma2_rn(__fmul2_rn(both(p.k30), r2), r2, __ffma2_rn(both(p.mxx), x2, q));
-}
-
 // G conj(Gamma_hat) of Gamma = pm conj(pk) - conj(pp) pk (corrected_from_apertures).
 // REFINE: the scale 1 / |Gamma| by rsqrtf and a Newton step, without which every
 // corrected value carries rsqrtf's rounding.
@@ -610,18 +596,6 @@ __device__ __forceinline__ float2 corrected_from_probes(float2 pm, float2 pp, fl
     gr *= inv;
     gi *= inv;
     return make_float2(fmaf(g.x, gr, g.y * gi), fmaf(g.y, gr, -g.x * gi));
-}
-
-// corrected_from_apertures in float32 chi, from the aperture pair a =
-// (A(q - k), A(q + k)) (evaluated, or of the per-geometry table).
-__device__ __forceinline__ float2 corrected_from_table(float2 a, float qx, float qy, float kx,
-                                                       float ky, float2 pk, float2 g, const Probe& p) {
-    const float2 chi = chi_pair(make_float2(qx - kx, qx + kx), make_float2(qy - ky, qy + ky), p);
-    float sm, cm, sp, cp;
-    __sincosf(chi.x, &sm, &cm);
-    __sincosf(chi.y, &sp, &cp);
-    return corrected_from_probes(make_float2(a.x * cm, -a.x * sm), make_float2(a.y * cp, -a.y * sp),
-                                 pk, g);
 }
 
 // C = G conj(Gamma_hat), Gamma = P(q-k) conj(P(k)) - conj(P(q+k)) P(k),
@@ -644,8 +618,7 @@ __device__ __forceinline__ float2 corrected(float qx, float qy, int r, int c, fl
         am = soft_aperture_fp64(qx64 - kx64, qy64 - ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
         ap = soft_aperture_fp64(qx64 + kx64, qy64 + ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
     }
-    if constexpr (CHI64) return corrected_from_apertures<CHI64>(dm, dp, am, ap, pk, g, p);
-    return corrected_from_table(make_float2(am, ap), qx, qy, kx, ky, pk, g, p);
+    return corrected_from_apertures<CHI64>(dm, dp, am, ap, pk, g, p);
 }
 
 // Probe constants of one candidate from the calibration (FP64 trig of phi12).
@@ -694,8 +667,6 @@ __host__ __device__ inline Probe make_probe_common(const qssb_calibration_t& cal
     p.mxx = (float)p.mxx_d;
     p.mxy = (float)p.mxy_d;
     p.myy = (float)p.myy_d;
-    p.mxy2 = (float)(2.0 * p.mxy_d);
-    p.k30 = (float)(0.5 * fl2 * cal.wavelength_A * cal.wavelength_A * (double)C30);
     p.quadratic = (C30 == 0.0f);
     return p;
 }

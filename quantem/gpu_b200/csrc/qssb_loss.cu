@@ -581,18 +581,11 @@ __device__ __forceinline__ float2 corrected_table_direct(float2 a, float qx, flo
                                                          const Probe& p) {
     const float m = ak * a.x;
     const float l = ak * a.y;
-    float2 chi;  // at q - k and q + k
-    if constexpr (CHI64) {
-        const Disp dm = displacement(qx - kx, qy - ky, p);
-        const Disp dp = displacement(qx + kx, qy + ky, p);
-        chi = make_float2(chi_value<CHI64>(dm.alpha2, dm.cos2, dm.sin2, p),
-                          chi_value<CHI64>(dp.alpha2, dp.cos2, dp.sin2, p));
-    } else {
-        chi = chi_pair(make_float2(qx - kx, qx + kx), make_float2(qy - ky, qy + ky), p);
-    }
+    const Disp dm = displacement(qx - kx, qy - ky, p);
+    const Disp dp = displacement(qx + kx, qy + ky, p);
     float sm, cm, sp, cp;
-    __sincosf(chi.x, &sm, &cm);
-    __sincosf(chi.y, &sp, &cp);
+    __sincosf(chi_value<CHI64>(dm.alpha2, dm.cos2, dm.sin2, p), &sm, &cm);
+    __sincosf(chi_value<CHI64>(dp.alpha2, dp.cos2, dp.sin2, p), &sp, &cp);
     // t1 = m (cm - i sm)(ck + i sk), t2 = l (cp + i sp)(ck - i sk)
     const float t1r = m * fmaf(cm, ek.x, sm * ek.y);
     const float t1i = m * fmaf(cm, ek.y, -sm * ek.x);
@@ -1250,9 +1243,7 @@ __device__ __forceinline__ void loss_rows_item(
         } else if constexpr (QUAD) {
             return corrected_quad<CHI64>(qx, qy, rr, c, eq, kq, gv, p);
         } else {
-            if constexpr (!CHI64) {
-                if (tab) return corrected_from_table(ov, qx, qy, kq.kx, kq.ky, pk, gv, p);
-            } else if (tab) {
+            if (tab) {
                 const Disp dm = displacement(qx - kq.kx, qy - kq.ky, p);
                 const Disp dp = displacement(qx + kq.kx, qy + kq.ky, p);
                 return corrected_from_apertures<CHI64>(dm, dp, ov.x, ov.y, pk, gv, p);
