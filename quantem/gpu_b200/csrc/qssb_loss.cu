@@ -1032,7 +1032,8 @@ __global__ void __launch_bounds__(256) k_loss_final_sq(const double* __restrict_
 //     own partial planes (column-major), so every element has one writer.
 constexpr int kL256 = 256;
 // Staging of one chunk. Twice the chunk halves the launches and their ramps
-// (16 candidates with C30 at 256^2: 18.5 ms with 32 MB, 17.0 with 64) and
+// (16 candidates with C30 at 256^2, their chi as a polynomial: 18.5 ms
+// with 32 MB, 17.0 with 64) and
 // still stays in L2. The quadratic loss at 256^2 keeps 32 MB: the persistent
 // launch holds three such slots in L2 and has the launch sequence's chunks.
 constexpr size_t kStageBudget = 64u << 20;
