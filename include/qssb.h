@@ -328,7 +328,10 @@ int qssb_object_noalloc(const float* g_half, const float* bf_geom, const float* 
                         const qssb_aberrations_t* ab, int32_t flags, float* object,
                         float* phase, void* stream);
 
-/* Workspace bytes needed by qssb_loss_batch for n_cand candidates. */
+/* Workspace bytes needed by qssb_loss_batch for n_cand candidates. A buffer
+ * sized with QSSB_FLAG_QUADRATIC or QSSB_FLAG_PERSISTENT serves batches without
+ * them too (at 256^2 with less staging than a buffer of their own: slower by
+ * a tenth, the same losses to float32 rounding). */
 int qssb_loss_workspace_bytes(const qssb_calibration_t* cal, int32_t n_cand, int32_t flags,
                               size_t* bytes);
 

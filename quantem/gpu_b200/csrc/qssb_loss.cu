@@ -1038,6 +1038,10 @@ constexpr int kL256 = 256;
 // launch holds three such slots in L2 and has the launch sequence's chunks.
 constexpr size_t kStageBudget = 64u << 20;
 constexpr size_t kStageBudgetQueue = 32u << 20;
+// Set by qssb_loss_batch_ex alone (callers' bit 7 is dropped): a buffer that
+// does not hold kStageBudget, one sized with QSSB_FLAG_QUADRATIC at 256^2 for
+// instance, takes the smaller staging.
+constexpr int kFlagSmallStaging = 1 << 7;
 // The persistent one-launch loss (k_loss_queue, QSSB_FLAG_PERSISTENT): 256^2,
 // half set, float32 chi, at most this many candidate groups (27 candidates each).
 constexpr int kQueueN = 256;
@@ -1624,15 +1628,14 @@ struct LossPlan {
 
 // Deterministic: about 296 CTAs in total (two per B200 SM), at least one BF
 // pixel each. N >= 256: the two-pass plan (n_chunks = its column interleave).
-static LossPlan plan_loss(int n, int n_bf, int n_cand, int chunks_req = 0, bool full = false,
-                          bool queue = false, bool quad = false) {
+static LossPlan plan_loss(int n, int n_bf, int n_cand, int chunks_req, bool full, bool queue,
+                          bool small) {
     LossPlan pl;
     pl.queue = false;
     pl.n_groups = 0;
     pl.n_phase_chunks = 0;
     pl.queue_bytes = 0;
     if (n >= kL256) {
-        const bool small = n == kQueueN && !full && (queue || quad);
         const TwoPassPlan tp = plan_two_pass(n, full, n_bf, n_cand, chunks_req,
                                              small ? kStageBudgetQueue : kStageBudget);
         pl.chunk_bf = tp.chunk_bf;
@@ -1711,6 +1714,14 @@ static LossPlan plan_loss(int n, int n_bf, int n_cand, int chunks_req = 0, bool 
     pl.eq_bytes = full ? 0 : sizeof(float2) * (size_t)n * n * n_cand;
     pl.stage_bytes = (pl.stage_bytes + 255) & ~(size_t)255;
     return pl;
+}
+
+// The plan of qssb_loss_batch.
+static LossPlan plan_loss_flags(int n, int n_bf, int n_cand, int flags) {
+    const bool queue = loss_queue_requested(n, flags);
+    const bool small = (n == kQueueN && (queue || (flags & QSSB_FLAG_QUADRATIC))) ||
+                       (flags & kFlagSmallStaging);
+    return plan_loss(n, n_bf, n_cand, flag_chunks(flags), false, queue, small);
 }
 
 static size_t loss_workspace(const LossPlan& pl) {
@@ -2027,9 +2038,7 @@ static int launch_loss(const float* g_half, const float* geom, const float* q_ro
                        const float* q_col, const qssb_calibration_t& cal,
                        const qssb_aberrations_t* cands, int n_cand, int flags, char* ws,
                        float* losses, float* mean_phase, const float2* overlap, cudaStream_t s) {
-    const LossPlan pl = plan_loss(N, cal.n_bf, n_cand, flag_chunks(flags), false,
-                                  loss_queue_requested(N, flags),
-                                  (flags & QSSB_FLAG_QUADRATIC) != 0);
+    const LossPlan pl = plan_loss_flags(N, cal.n_bf, n_cand, flags);
     float* part = reinterpret_cast<float*>(ws);
     double* var = reinterpret_cast<double*>(ws + pl.part_bytes);
     float2* eq = reinterpret_cast<float2*>(ws + pl.part_bytes + pl.var_bytes);
@@ -2403,7 +2412,7 @@ static int launch_loss_full(const float* g_half, const float* geom, const float*
                             const float* q_col, const qssb_calibration_t& cal,
                             const qssb_full_aberrations_t* cands, int n_cand, int chunks, char* ws,
                             float* losses, float* mean_phase, cudaStream_t s) {
-    const LossPlan pl = plan_loss(N, cal.n_bf, n_cand, chunks, true);
+    const LossPlan pl = plan_loss(N, cal.n_bf, n_cand, chunks, true, false, false);
     float* part = reinterpret_cast<float*>(ws);
     double* var = reinterpret_cast<double*>(ws + pl.part_bytes);
     if constexpr (N >= kL256) {
@@ -2467,10 +2476,7 @@ extern "C" int qssb_loss_workspace_bytes(const qssb_calibration_t* cal, int32_t 
     if (n != 64 && n != 128 && n != 256 && n != 512 && n != 1024)
         return set_error(QSSB_ERR_UNSUPPORTED,
                          "qssb_loss_batch: scan size must be 64, 128, 256, 512 or 1024");
-    const LossPlan pl =
-        plan_loss(n, cal->n_bf, n_cand, flag_chunks(flags), false, loss_queue_requested(n, flags),
-                  (flags & QSSB_FLAG_QUADRATIC) != 0);
-    *bytes = loss_workspace(pl);
+    *bytes = loss_workspace(plan_loss_flags(n, cal->n_bf, n_cand, flags & ~kFlagSmallStaging));
     return QSSB_OK;
 }
 
@@ -2539,10 +2545,15 @@ extern "C" int qssb_loss_batch_ex(const float* g_half, const float* bf_geom, con
     if (!g_half || !bf_geom || !q_row || !q_col || !candidates || !workspace || !losses)
         return set_error(QSSB_ERR_INVALID, "qssb_loss_batch: null pointer");
     size_t need = 0;
+    flags &= ~kFlagSmallStaging;
     rc = qssb_loss_workspace_bytes(cal, n_cand, flags, &need);
     if (rc) return rc;
-    if (workspace_bytes < need)
-        return set_error(QSSB_ERR_WORKSPACE, "qssb_loss_batch: workspace too small");
+    if (workspace_bytes < need) {
+        flags |= kFlagSmallStaging;
+        if (workspace_bytes <
+            loss_workspace(plan_loss_flags(cal->scan_rows, cal->n_bf, n_cand, flags)))
+            return set_error(QSSB_ERR_WORKSPACE, "qssb_loss_batch: workspace too small");
+    }
     if (((uintptr_t)workspace & 255u) != 0)
         return set_error(QSSB_ERR_INVALID, "qssb_loss_batch: workspace must be 256-byte aligned");
     const bool sym = !(flags & QSSB_FLAG_FULL_PLANE);
@@ -2575,7 +2586,7 @@ extern "C" int qssb_loss_full_workspace_bytes(const qssb_calibration_t* cal, int
     if (n != 64 && n != 128 && n != 256 && n != 512 && n != 1024)
         return set_error(QSSB_ERR_UNSUPPORTED,
                          "qssb_loss_batch_full: scan size must be 64, 128, 256, 512 or 1024");
-    const LossPlan pl = plan_loss(n, cal->n_bf, n_cand, flag_chunks(flags), true);
+    const LossPlan pl = plan_loss(n, cal->n_bf, n_cand, flag_chunks(flags), true, false, false);
     *bytes = loss_workspace(pl);
     return QSSB_OK;
 }

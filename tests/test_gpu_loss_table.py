@@ -17,6 +17,7 @@ table-free kernel, and the backend's table switch are checked.
 """
 from __future__ import annotations
 
+import ctypes
 import math
 
 import numpy as np
@@ -24,7 +25,7 @@ import pytest
 import torch
 
 from oracle import ssb_oracle as so
-from quantem.gpu_b200 import B200SSBBackend, ops
+from quantem.gpu_b200 import B200SSBBackend, _lib, ops
 from quantem.gpu_b200._lib import (QSSB_FLAG_CHI_FP64, QSSB_FLAG_PERSISTENT,
                                    QSSB_FLAG_QUADRATIC)
 from recipes import disk_input, synthetic_plain_32
@@ -332,3 +333,32 @@ def test_persistent_launch_cancel_flag_gives_nan_without_hanging(case256):
         np.testing.assert_array_equal(run(), want)
     finally:
         ops.set_cancel_flag(None)
+
+
+def _loss_in(case256, cands, flags, nbytes):
+    """Losses of cands in a workspace of nbytes, by the C entry itself."""
+    _, cal, d = case256
+    buf = torch.empty(nbytes, dtype=torch.uint8, device=DEV)
+    out = torch.empty(cands.shape[0], dtype=torch.float32, device=DEV)
+    ops._call("qssb_loss_batch", DEV, *(ops._ptr(d[k]) for k in ("g", "geom", "q_row", "q_col")),
+              ctypes.byref(cal), ops._ptr(cands), cands.shape[0], flags, ops._ptr(buf), nbytes,
+              ops._ptr(out), None, ops._stream(out))
+    return out
+
+
+@pytest.mark.parametrize("n_cand,sized", [
+    (16, QSSB_FLAG_QUADRATIC), (64, QSSB_FLAG_QUADRATIC), (64, QSSB_FLAG_PERSISTENT),
+    (460, QSSB_FLAG_QUADRATIC | QSSB_FLAG_PERSISTENT)])  # 18 groups: more than one launch takes
+def test_a_buffer_sized_for_one_kind_of_batch_serves_the_other(case256, n_cand, sized):
+    """C30 batches in a buffer that was sized with QSSB_FLAG_QUADRATIC or
+    QSSB_FLAG_PERSISTENT, whose staging is smaller: other chunks of BF pixels,
+    so the sums' order differs (float32 sums of 27 values over few chunks:
+    1e-6); a byte less is refused."""
+    cal = case256[1]
+    cands = _rows(n_cand, seed=n_cand, c30=True)
+    small, own = ops.loss_workspace_bytes(cal, n_cand, sized), ops.loss_workspace_bytes(cal, n_cand)
+    got = _loss_in(case256, cands, 0, small)
+    torch.testing.assert_close(got, _loss_in(case256, cands, 0, own), rtol=1e-6, atol=0)
+    least = ops.loss_workspace_bytes(cal, n_cand, QSSB_FLAG_QUADRATIC)
+    with pytest.raises(_lib.QssbError, match="workspace too small"):
+        _loss_in(case256, cands, 0, least - 1)
