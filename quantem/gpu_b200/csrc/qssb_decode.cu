@@ -537,8 +537,9 @@ __global__ void k_bslz4_chunk_sizes(const uint8_t* __restrict__ scratch, int n_c
 
 // One warp per (chunk, block): the block's slot to its place in the chunk
 // (the sizes of the chunk's earlier blocks summed by the lanes), 16 bytes a
-// lane on the destination's alignment, the source words funnel-shifted. The
-// first block's warp writes the chunk header, the last one's the raw leftovers.
+// lane on the destination's alignment, the source words funnel-shifted (by
+// bytes where a caller's scratch does not start on a word). The first block's
+// warp writes the chunk header, the last one's the raw leftovers.
 constexpr int kPackWarps = 8;
 __global__ void __launch_bounds__(32 * kPackWarps) k_bslz4_pack(
     const uint8_t* __restrict__ scratch, const uint16_t* __restrict__ frames, long long n_items,
@@ -565,7 +566,7 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_bslz4_pack(
     const int len = n_blocks ? 4 + (int)be32(slot) : 0;
     const int head = min(len, (int)((16u - ((uintptr_t)dst & 15u)) & 15u));
     if (lane < head) dst[lane] = slot[lane];
-    const int n_vec = (len - head) >> 4;
+    const int n_vec = ((uintptr_t)slot & 3u) == 0 ? (len - head) >> 4 : 0;
     const int shift = 8 * (head & 3);
     const uint32_t* words = reinterpret_cast<const uint32_t*>(slot) + (head >> 2);
     uint4* out = reinterpret_cast<uint4*>(dst + head);
@@ -576,8 +577,7 @@ __global__ void __launch_bounds__(32 * kPackWarps) k_bslz4_pack(
         out[t] = make_uint4(__funnelshift_r(w[0], w1, shift), __funnelshift_r(w1, w2, shift),
                             __funnelshift_r(w2, w3, shift), __funnelshift_r(w3, w4, shift));
     }
-    const int done = head + 16 * n_vec;
-    if (done + lane < len) dst[done + lane] = slot[done + lane];
+    for (int j = head + 16 * n_vec + lane; j < len; j += 32) dst[j] = slot[j];
     if (i + 1 < n_blocks) return;
     const uint16_t* frame = frames + (size_t)c * n_elem;
     for (long long j = n8 + lane; j < n_elem; j += 32) {

@@ -6,6 +6,7 @@ reference's readers; malformed chunks are reported per chunk without a
 fault; decoded counts reconstruct exactly as the originals."""
 from __future__ import annotations
 
+import ctypes
 import struct
 
 import numpy as np
@@ -14,7 +15,7 @@ import torch
 
 from oracle import bslz4_oracle as bo
 from oracle.ref_cuda import build_bslz4
-from quantem.gpu_b200 import SSB
+from quantem.gpu_b200 import SSB, _lib, ops
 from quantem.gpu_b200.decode import decode_bslz4, encode_bslz4, from_chunks
 from quantem.gpu_b200.synthetic import CONFIGS, generate
 
@@ -188,3 +189,31 @@ def test_encoder_writes_the_serial_search_bytes(shape, kind):
         want.append(chunk + f[n // 8 * 8:].tobytes())
     assert offsets.cpu().tolist() == [0, len(want[0]), len(want[0]) + len(want[1])]
     assert packed.cpu().numpy().tobytes() == b"".join(want)
+
+
+@pytest.mark.parametrize("elements", [1, 7, 8, 4104, 12291])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3, 4, 16])
+def test_pack_takes_scratch_and_output_at_any_address(elements, shift):
+    """The C entries with scratch (and, the other way round, packed bytes)
+    ``shift`` bytes into a buffer, down to chunks of raw elements alone."""
+    frames = _frames(3, (elements, 1), seed=elements)
+    t = torch.as_tensor(frames, device=DEV)
+    want, want_offsets = bo.pack([bo.encode_chunk(f) for f in frames])
+    nbytes = ctypes.c_size_t(0)
+    _lib.check(_lib.load().qssb_encode_bslz4_scratch_bytes(3, 2 * elements, ctypes.byref(nbytes)))
+    scratch = torch.empty(nbytes.value + 64, dtype=torch.uint8, device=DEV)[shift:]
+    sizes = torch.empty(3, dtype=torch.int64, device=DEV)
+    ops._call("qssb_encode_bslz4_u16", DEV, ops._ptr(t), 3, 2 * elements, ops._ptr(scratch),
+              ops._ptr(sizes), ops._stream(t))
+    offsets = torch.cumsum(sizes, 0) - sizes
+    packed = torch.zeros(int(sizes.sum()) + 32, dtype=torch.uint8, device=DEV)[16 - shift:]
+    ops._call("qssb_pack_bslz4", DEV, ops._ptr(scratch), ops._ptr(t), 3, 2 * elements,
+              ops._ptr(offsets), ops._ptr(packed), ops._stream(t))
+    host, offs = packed.cpu().numpy(), offsets.cpu().tolist()
+    end = offs[1:] + [int(sizes.sum())]
+    assert not host[end[-1]:].any()
+    for f, a, b in zip(frames, offs, end):
+        np.testing.assert_array_equal(bo.decode_chunk(host[a:b].tobytes()).reshape(f.shape), f)
+    if elements < 8:  # raw elements only: the same bytes from any encoder
+        assert offs == want_offsets.tolist()
+        np.testing.assert_array_equal(host[:end[-1]], want)
