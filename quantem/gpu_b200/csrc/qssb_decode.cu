@@ -17,7 +17,7 @@
 // L1, all lanes copy literals and matches - a match byte j reads
 // out[op - off + j mod off], so overlapping matches need no serial copy) and
 // bit-unshuffles the block with 8x8 bit transposes straight into the u16
-// frame (16-byte stores). A malformed chunk sets status[c] (the block is
+// frame (32-byte stores where the frames allow it). A malformed chunk sets status[c] (the block is
 // zero-filled); nothing traps.
 // Encode: a warp per block makes the same transposes forward and the greedy
 // LZ4 of a serial search (32 positions a step, a 4096-entry hash table in
@@ -297,8 +297,8 @@ __device__ __forceinline__ void unshuffle_store(const uint8_t* planes, int cnt, 
 // W warps per chunk, which share nothing: each walks the block chain itself
 // (every lane reads the same words, prefetched into L1), first to the end to
 // check it, then along the blocks it takes. W = 1 where the chunks fill the
-// chip: a frame's blocks differ widely in cost, and the warps of a larger CTA
-// hold their shared memory until its slowest is done. Bound by the latency
+// chip (decode_one_warp): a frame's blocks differ widely in cost, and the warps
+// of a larger CTA hold their shared memory until its slowest is done. Bound by the latency
 // and issue of the per-sequence chain. 16384 frames of 128 x 128 counts: the
 // call 0.49 ms, against 1.09 with four warps a chunk, one thread's chain
 // walk, one sequence parsed at a time, matches copied and planes read by bytes.
@@ -593,6 +593,27 @@ static int chunk_blocks(long long chunk_bytes) {
     return (int)((n8 + kBlockElems - 1) / kBlockElems);
 }
 
+// One warp per chunk or four. An SM holds 24 one-warp CTAs (8 KB, and 1 KB of
+// the system's, each) or 6 four-warp CTAs, the same 24 blocks, so the choice is
+// between idle warps and chunks left waiting. Four warps a chunk against one,
+// call, us (counts of dose 1000):
+//   1 block (64 x 64):    900 chunks  51.3 / 30.7, 128 to 512 chunks equal;
+//   3 blocks (110 x 110): 888 chunks  47.2 / 64.7, 900 (a second wave of
+//                         four-warp CTAs) 67.4 / 65.5, 1860  105 / 84;
+//   4 blocks (128 x 128): 1776 chunks 69.8 / 76.1, 1924 86.4 / 83.8,
+//                         8192  295 / 243;
+//   6 blocks (144 x 144): 1924 chunks 95 / 101, 4096 176 / 184; sparser counts
+//                         up to 14% for four warps, denser ones 7% for one;
+//   7 blocks (160 x 160): 1924 chunks 103 / 121, 4096 189 / 217; 16 blocks
+//                         4096 chunks 442 / 545: one warp's chain through many
+//                         blocks of a chunk outlasts the others.
+static bool decode_one_warp(int n_chunks, int n_blocks) {
+    const int sms = device_sm_count();
+    if (n_blocks <= 1) return true;
+    if (n_blocks <= 3) return n_chunks > 6 * sms;
+    return n_blocks <= 6 && n_chunks >= 13 * sms;
+}
+
 static int check_chunk_bytes(long long chunk_bytes, const char* who) {
     if (chunk_bytes < 2 || (chunk_bytes & 1) || chunk_bytes / 2 / kBlockElems >= kMaxBlocks)
         return set_error(QSSB_ERR_INVALID, who);
@@ -618,8 +639,7 @@ extern "C" int qssb_decode_bslz4_u16(const uint8_t* compressed, int64_t compress
             chunk_bytes, out, status);
         note_launch();
     };
-    // 27 warps of 8 KB fit an SM; fewer chunks than half of that take four warps each
-    if (n_chunks >= 13 * device_sm_count())
+    if (decode_one_warp(n_chunks, chunk_blocks(chunk_bytes)))
         launch(k_decode_bslz4_u16<1>, 1);
     else
         launch(k_decode_bslz4_u16<kDecWarps>, kDecWarps);
