@@ -189,6 +189,7 @@ def test_encoder_writes_the_serial_search_bytes(shape, kind):
         want.append(chunk + f[n // 8 * 8:].tobytes())
     assert offsets.cpu().tolist() == [0, len(want[0]), len(want[0]) + len(want[1])]
     assert packed.cpu().numpy().tobytes() == b"".join(want)
+    np.testing.assert_array_equal(decode_bslz4(packed, offsets, shape).cpu().numpy(), frames)
 
 
 @pytest.mark.parametrize("elements", [1, 7, 8, 4104, 12291])
@@ -217,3 +218,144 @@ def test_pack_takes_scratch_and_output_at_any_address(elements, shift):
     if elements < 8:  # raw elements only: the same bytes from any encoder
         assert offs == want_offsets.tolist()
         np.testing.assert_array_equal(host[:end[-1]], want)
+
+
+def _many():
+    """More chunks than the decoder gives four warps each."""
+    return 13 * torch.cuda.get_device_properties(DEV).multi_processor_count + 1
+
+
+def _decode_raw(chunks, elements, n):
+    """(frames, statuses) of the first n of the chunks, repeated in turn."""
+    picked = [chunks[i % len(chunks)] for i in range(n)]
+    data, offsets = bo.pack(picked)
+    comp, offs = torch.as_tensor(data, device=DEV), torch.as_tensor(offsets, device=DEV)
+    out = torch.full((n, elements), 0x5a5a, dtype=torch.uint16, device=DEV)
+    status = torch.full((n,), -1, dtype=torch.int32, device=DEV)
+    ops._call("qssb_decode_bslz4_u16", DEV, ops._ptr(comp), comp.numel(), ops._ptr(offs), n,
+              2 * elements, ops._ptr(out), ops._ptr(status), ops._stream(out))
+    return out.cpu().numpy(), status.cpu().numpy()
+
+
+def _sequence(lit: bytes, off=None, ml=4) -> bytes:
+    """One LZ4 sequence (the last of a block without an offset)."""
+    def ext(x):
+        return b"\xff" * ((x - 15) // 255) + bytes([(x - 15) % 255]) if x >= 15 else b""
+
+    head = bytes([min(len(lit), 15) << 4 | (0 if off is None else min(ml - 4, 15))])
+    body = head + ext(len(lit)) + lit
+    return body if off is None else body + struct.pack("<H", off) + ext(ml - 4)
+
+
+OFFSETS = (1, 2, 3, 5, 31, 32, 33, 100, 127, 128, 129, 255, 511, 512, 513, 700)
+LENGTHS = (4, 18, 19, 32, 33, 127, 131, 260, 515, 700, 6000)
+
+
+def _blocks(rng):
+    """LZ4 blocks of 8192 bytes with every offset and match length above at
+    every output alignment, between literal runs of every token form, so that
+    tokens fall anywhere in the 32 bytes that the decoder parses at once."""
+    wanted = [(o, m, a) for o in OFFSETS for m in LENGTHS for a in range(4)]
+    rng.shuffle(wanted)
+    blocks, src, op = [], b"", 0
+    for off, ml, align in wanted:
+        for _ in range(2):
+            lit = max(off - op, 0) + int(rng.choice([0, 0, 1, 3, 14, 15, 16, 40]))
+            lit += (align - op - lit) % 4
+            if op + lit + ml <= 8192:
+                break
+            blocks.append(src + _sequence(rng.bytes(8192 - op)))
+            src, op = b"", 0
+        src += _sequence(rng.bytes(lit), off, ml)
+        op += lit + ml
+    return blocks + [src + _sequence(rng.bytes(8192 - op))]
+
+
+def _tail(rng, nbytes):
+    """A block of a few bytes: literals, a short match where it fits, the rest."""
+    if nbytes < 24:
+        return _sequence(rng.bytes(nbytes))
+    return _sequence(rng.bytes(5), 3, 9) + _sequence(rng.bytes(nbytes - 14))
+
+
+def _chunk(blocks, raw=b"", total=None):
+    body = b"".join(struct.pack(">I", len(b)) + b for b in blocks)
+    return struct.pack(">QI", total, 8192) + body + raw
+
+
+@pytest.mark.parametrize("elements", [4160, 4104, 4127])  # 32-byte, 16-byte and 2-byte stores
+@pytest.mark.parametrize("many", [False, True])  # four warps a chunk, one
+def test_matches_of_every_offset_length_and_alignment(elements, many):
+    rng = np.random.default_rng(elements)
+    chunks = [_chunk([b, _tail(rng, 2 * (elements // 8 * 8 - 4096))], rng.bytes(2 * (elements % 8)),
+                     2 * elements) for b in _blocks(rng)]
+    assert len(chunks) > 40
+    want = np.stack([bo.decode_chunk(c) for c in chunks])
+    n = _many() if many else len(chunks)
+    got, status = _decode_raw(chunks, elements, n)
+    assert not status.any()
+    np.testing.assert_array_equal(got, want[np.arange(n) % len(chunks)])
+
+
+@pytest.mark.parametrize("elements", [8, 15, 23])
+def test_chunks_of_one_short_block(elements):
+    rng = np.random.default_rng(elements)
+    chunks = [_chunk([_tail(rng, 2 * (elements // 8 * 8))], rng.bytes(2 * (elements % 8)),
+                     2 * elements) for _ in range(33)]
+    want = np.stack([bo.decode_chunk(c) for c in chunks])
+    got, status = _decode_raw(chunks, elements, 33)
+    assert not status.any()
+    np.testing.assert_array_equal(got, want)
+
+
+RUN = _sequence(b"ab", 1, 8170)  # 8172 bytes of output
+MALFORMED = {
+    "no bytes": b"",
+    "literal length cut off": b"\xf0\xff\xff",
+    "match length cut off": b"\x1fa\x01\x00\xff",
+    "literals cut off": b"\xe0abc",
+    "offset cut off": _sequence(b"abcd", 2, 9) + b"\x10a\x01",
+    "offset 0": _sequence(b"abc", 0, 9) + _sequence(b"x" * 8180),
+    "offset 0 of a long match": _sequence(b"abc", 0, 99) + _sequence(b"x" * 8090),
+    "offset before the output": _sequence(b"abc", 4, 9) + _sequence(b"x" * 8180),
+    "offset before the output, long": _sequence(b"abc", 9, 99) + _sequence(b"x" * 8090),
+    "match past the output": RUN + _sequence(b"12345678", 2, 13) + _sequence(b"x"),
+    "long match past the output": _sequence(b"ab", 1, 9000) + _sequence(b"x"),
+    "literals past the output": _sequence(b"x" * 8193),
+    "literals past the output, short": RUN + _sequence(b"x" * 14, 1, 9) + _sequence(b"x"),
+    "ends with a match": RUN + _sequence(b"12345678", 2, 12),
+    "ends with a long match": _sequence(b"ab", 1, 8190),
+    "ends with the parsed window": b"".join(_sequence(b"a", 1, 4) for _ in range(8)),
+    "too short": RUN + _sequence(b"x" * 19),
+    "goes on when full": RUN + _sequence(b"x" * 8, 1, 12) + _sequence(b"", 1, 4) + _sequence(b""),
+}
+
+
+@pytest.mark.parametrize("many", [False, True])
+def test_malformed_blocks_in_both_kernels(many):
+    """Between well-formed chunks: status 3, the bad block zero, the rest kept."""
+    rng = np.random.default_rng(8)
+    good = _blocks(rng)
+    kinds = list(MALFORMED)
+    for k in kinds:
+        with pytest.raises(ValueError):
+            bo.lz4_decompress(MALFORMED[k], 8192)
+    tail = _tail(rng, 128)
+    rest = bo.bitunshuffle(bo.lz4_decompress(tail, 128), 64, np.uint16)
+    chunks, want = [], []
+    for i, k in enumerate(kinds):
+        for block in (MALFORMED[k], good[i]):
+            chunks.append(_chunk([block, tail], total=2 * 4160))
+            head = (np.zeros(4096, np.uint16) if block is MALFORMED[k]
+                    else bo.bitunshuffle(bo.lz4_decompress(block, 8192), 4096, np.uint16))
+            want.append(np.concatenate([head, rest]))
+    # the chain and the header: the whole chunk is zero
+    for bad, code in ((chunks[1][:-1], 2), (_corrupt(chunks[1], "header"), 1), (b"\x00" * 11, 1)):
+        chunks.append(bad)
+        want.append(np.zeros(4160, np.uint16))
+    codes = np.array([3, 0] * len(kinds) + [2, 1, 1])
+    n = _many() if many else len(chunks)
+    got, status = _decode_raw(chunks, 4160, n)
+    at = np.arange(n) % len(chunks)
+    assert [int(s) for s in status] == codes[at].tolist()
+    np.testing.assert_array_equal(got, np.stack(want)[at])
