@@ -1065,9 +1065,14 @@ static bool loss_queue_requested(int n, int flags) {
 __host__ __device__ constexpr int row_warps(int n) { return n >= 1024 ? 8 : (n == 256 ? 8 : 16); }
 __host__ __device__ constexpr int row_min_ctas(int n) { return n == 256 ? 3 : 1; }
 // The 14-term chi's CTA starts with FP64 work (its coefficients, P(k)), shared
-// by four rows a warp at 256^2 (2 candidates of 1789 BF pixels: 9.0 ms with one
-// row a warp, 6.9 with four); the half set measured the same either way.
-__host__ __device__ constexpr int rows_per_warp(int n, bool full) { return full && n == 256 ? 4 : 1; }
+// by four rows a warp up to 512^2. One row a warp against four, with the plan's
+// chunk that fills the waves: 2 candidates of 1781 BF pixels at 256^2 8.6 / 6.8
+// ms, of 437 at 512^2 9.2 / 7.4 (9 candidates 40.1 / 31.9); at 1024^2, where a
+// row is 32 values a lane, 1 candidate of 109 BF pixels 7.3 / 7.5, 4 candidates
+// 29.9 / 28.9. The half set has no such start: with four rows at 256^2 a batch
+// with C30 takes 8% longer (16 candidates: 19.2 / 20.8 ms), a quadratic one 12%
+// (19.5 / 21.7) and from a full group of 27 on 6% less (30.3 / 28.4).
+__host__ __device__ constexpr int rows_per_warp(int n, bool full) { return full && n <= 512 ? 4 : 1; }
 __host__ __device__ constexpr int row_load_batch(int n) { return n == 256 ? 4 : 8; }
 __host__ __device__ constexpr int col_tile(int n) { return n >= 1024 ? 8 : 16; }
 
@@ -1129,10 +1134,13 @@ static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chu
     const size_t per_bf = sizeof(float2) * (size_t)(full ? n : n / 2 + 1) * n;
     long long c = (long long)(budget / (per_bf * (size_t)group));
     if (c < 1) c = 1;
-    if (full && n == 256) {
+    if (rows_per_warp(n, full) > 1) {
         // the chunk, from the budget down to half of it, whose row pass fills its
-        // waves best (an item is 32 rows, so a last wave is a larger share)
-        const long long items = (long long)TwoPass<256, true>::row_ctas * group;
+        // waves best (an item is 32 or 64 rows, so a last wave is a larger share:
+        // 2 candidates at 256^2 7.4 ms with the budget's chunk, 6.8 with this one,
+        // 9 at 512^2 40.5 and 31.9)
+        const int ctas = n == 256 ? TwoPass<256, true>::row_ctas : TwoPass<512, true>::row_ctas;
+        const long long items = (long long)ctas * group;
         const long long rslots = 148LL * row_min_ctas(n);
         double best = 0.0;
         for (long long k = c, kmin = (c + 1) / 2; k >= kmin; --k) {

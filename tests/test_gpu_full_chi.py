@@ -165,3 +165,21 @@ def test_paired_evaluation_matches_the_fp64_chi_kernel(chunks, det_sampling):
     err = so.wrapped_phase_error(phase.cpu().numpy(), phase64.cpu().numpy())
     assert float(np.sqrt(np.mean(err ** 2))) < 2e-5
     be.close()
+
+
+def test_512_rows_in_groups_match_the_symmetric_path():
+    """k_loss_rows<512, FULL> (four rows a warp, chunks that fill its waves)
+    with C10, C12 and C30 only, against the half-set kernels, for a group of
+    candidates and one beyond it; 27 BF pixels, float32 sums: 2e-6."""
+    counts = disk_input(123, scan=(512, 512))
+    be = B200SSBBackend(torch.as_tensor(counts, device=DEV), semiangle=21.4, scan_sampling=0.5,
+                        det_sampling=1.0, voltage_kV=300, bf_radius=3)
+    for n in (1, 10):
+        rng = np.random.default_rng(n)
+        mags, angs = np.zeros((n, 14)), np.zeros((n, 14))
+        mags[:, 0], mags[:, 1] = rng.uniform(-150, 150, n), rng.uniform(0, 60, n)
+        angs[:, 1], mags[:, 4] = rng.uniform(-1.5, 1.5, n), rng.uniform(0, 5e4, n)
+        got = be.variance_loss_batch_full(mags, angs)
+        want = be.variance_loss_batch(mags[:, 0], mags[:, 1], angs[:, 1], mags[:, 4])
+        torch.testing.assert_close(got, want, rtol=2e-6, atol=0)
+    be.close()
