@@ -925,14 +925,13 @@ extern "C" int qssb_gather_bf_columns_2d(const uint16_t* counts, int64_t n_frame
 //     per pair), forward warp FFT, split into the two real rows' spectra
 //     X_2j(c) = (Z(c) + conj Z(-c)) / 2, X_2j+1(c) = (Z(c) - conj Z(-c)) / 2i,
 //     c = 0..N/2, written to G[b][row][c];
-//   k_scan_cols<N>: T columns of G[b] staged in shared memory (odd pitch:
-//     the T columns of one row land on distinct banks), forward warp FFT of
-//     each column along the rows, written back in place.
+//   k_scan_cols_p<N>: strips of T columns of G[b] staged in shared memory
+//     (strip_pitch), forward warp FFT of each column along the rows, written
+//     back in place.
 template <int N>
 struct ScanLines {
     static constexpr int H = N / 2 + 1;
     static constexpr int kWarps = N >= 1024 ? 4 : 8;       // row pairs per block
-    static constexpr int kTile = N >= 1024 ? 8 : 16;       // columns per block
     // persistent column pass: columns per strip (one warp each) and CTAs per
     // SM. At 256 three 8-warp CTAs per SM (0.63 ms for the two scan passes of
     // 1783 BF pixels against 0.71 with one 16-warp CTA); at 512 and 1024 the
@@ -940,9 +939,7 @@ struct ScanLines {
     static constexpr int kTileP = N >= 1024 ? 8 : (N == 256 ? 8 : 16);
     static constexpr int kCtasP = N == 256 ? 3 : 1;
     static constexpr int kScratch = warp_fft_scratch<N>();  // >= N: also holds a line
-    static constexpr int P = kScratch | 1;                  // column pitch, odd mod 16
     static constexpr size_t rows_smem = sizeof(float2) * ((size_t)kWarps * kScratch + N);
-    static constexpr size_t cols_smem = sizeof(float2) * ((size_t)kTile * P + N);
 };
 
 // Place of a spectrum's element in its shared line. The warp FFT leaves a lane
@@ -1005,52 +1002,6 @@ __global__ void __launch_bounds__(32 * ScanLines<N>::kWarps) k_scan_rows(
         const float2 m = x[line_place<N>((N - c) & (N - 1))];
         g0[c] = make_float2(0.5f * (z.x + m.x), 0.5f * (z.y - m.y));
         g1[c] = make_float2(0.5f * (z.y + m.y), -0.5f * (z.x - m.x));
-    }
-}
-
-// Columns: T columns of G[b] staged in shared memory, one warp FFT per
-// column (the column's own line is the transpose scratch), written back.
-template <int N>
-__global__ void __launch_bounds__(256) k_scan_cols(int n_bf, float2* __restrict__ g_half) {
-    using L = ScanLines<N>;
-    constexpr int P = L::P;
-    constexpr int T = L::kTile;
-    constexpr int H = L::H;
-    constexpr int RPL = N / 32;
-    extern __shared__ float2 scan_cols_smem[];
-    float2* tile = scan_cols_smem;
-    float2* tw = tile + T * P;
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int warp = tid >> 5;
-    fill_twiddles<N>(tw, tid, 256);
-    const int b = blockIdx.x;
-    const int c0 = blockIdx.y * T;
-    const int nc = min(T, H - c0);
-    if (b >= n_bf) return;  // uniform per block: before any barrier
-    float2* g = g_half + (size_t)b * N * H;
-    for (int e = tid; e < N * T; e += 256) {
-        const int r = e / T;
-        const int c = e - r * T;
-        if (c < nc) tile[c * P + r] = g[(size_t)r * H + c0 + c];
-    }
-    __syncthreads();
-    for (int c = warp; c < nc; c += 8) {
-        float2* line = tile + c * P;
-        float2 v[RPL];
-#pragma unroll
-        for (int t = 0; t < RPL; ++t) v[t] = line[lane + 32 * t];
-        __syncwarp();
-        warp_fft<N, -1>(v, line, tw, lane);
-#pragma unroll
-        for (int j = 0; j < RPL; ++j) line[warp_fft_index<N>(lane, j)] = v[j];
-        __syncwarp();
-    }
-    __syncthreads();
-    for (int e = tid; e < N * T; e += 256) {
-        const int r = e / T;
-        const int c = e - r * T;
-        if (c < nc) g[(size_t)r * H + c0 + c] = tile[c * P + r];
     }
 }
 
@@ -1149,8 +1100,6 @@ static int launch_scan_lines(const uint16_t* columns, int n_bf, float* g_half, i
     { k_scan_rows<N><<<dim3(n_bf, (N / 2 + L::kWarps - 1) / L::kWarps), 32 * L::kWarps,
                      L::rows_smem, s>>>(columns, n_bf, g); note_launch(); }
     CUDA_TRY(cudaGetLastError());
-    CUDA_TRY(cudaFuncSetAttribute(k_scan_cols<N>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)L::cols_smem));
     int rc = QSSB_OK;
     if constexpr (N == 256) {
         switch (variant) {
@@ -1165,13 +1114,11 @@ static int launch_scan_lines(const uint16_t* columns, int n_bf, float* g_half, i
             case 3: rc = launch_scan_cols_p<N, 8, 2>(n_bf, g, s); break;
             default: rc = launch_scan_cols_p<N, L::kTileP, L::kCtasP>(n_bf, g, s); break;
         }
-    } else if constexpr (N >= 1024) {
+    } else {
         switch (variant) {
             case 2: rc = launch_scan_cols_p<N, 4, 2>(n_bf, g, s); break;
             default: rc = launch_scan_cols_p<N, L::kTileP, L::kCtasP>(n_bf, g, s); break;
         }
-    } else {
-        { k_scan_cols<N><<<dim3(n_bf, (L::H + L::kTile - 1) / L::kTile), 256, L::cols_smem, s>>>(n_bf, g); note_launch(); }
     }
     if (rc) return rc;
     CUDA_TRY(cudaGetLastError());
