@@ -40,9 +40,11 @@ extern "C" {
 #define QSSB_FLAG_PERSISTENT 8    /* qssb_loss_batch at 256^2 (float32 chi): one persistent
                                      launch runs every row and column item of the batch
                                      instead of a row and a column launch per BF chunk
-                                     (the same plan; the same bits with
-                                     QSSB_FLAG_QUADRATIC, float32 rounding without;
-                                     within 3% of the sequence's time) */
+                                     (few kernels in a graph; the same bits with
+                                     QSSB_FLAG_QUADRATIC, float32 rounding without.
+                                     Slower than the launches: three scans' sweep of
+                                     64 candidates each takes 10% longer with C30, 7%
+                                     with QSSB_FLAG_QUADRATIC) */
 /* Tile-shape variant (another tuning knob): bits 8..11 of flags. qssb_object
  * on the quadratic-chi path: 1 = 2 adjacent frequencies per thread, 2 or 0
  * (the default) = 4, 3 = 8. Results agree to float32 rounding across
@@ -386,9 +388,9 @@ int qssb_overlap_table(const float* bf_geom, const float* q_row, const float* q_
  * Nyquist-line parts transformed on their own) with the apertures read from
  * the table: for QSSB_FLAG_QUADRATIC batches through the factorised overlap,
  * otherwise (C30) through the direct probe phases. With a table and 256 .. 1024
- * scans, the row pass of QSSB_FLAG_QUADRATIC batches (without
- * QSSB_FLAG_CHI_FP64) reads the apertures instead of evaluating them; other
- * batches there ignore the table. The workspace is the same. The reduction
+ * scans, the row pass reads the apertures instead of evaluating them
+ * (QSSB_FLAG_QUADRATIC batches with QSSB_FLAG_CHI_FP64 ignore the table there).
+ * The workspace is the same. The reduction
  * order is fixed for a given plan; the result differs from the table-free path
  * by float32 rounding only. */
 int qssb_loss_batch_ex(const float* g_half, const float* bf_geom, const float* q_row,
@@ -424,8 +426,8 @@ int qssb_loss_full_workspace_bytes(const qssb_calibration_t* cal, int32_t n_cand
 /* qssb_loss_batch with the 14-term chi: replaces reconstruct_full /
  * reconstruct_full_with_loss (engine.py:1244-1458; the reference raises
  * NotImplementedError at 128, engine.py:1276-1280, 1373-1377 - this entry
- * serves 64, 128 and 256). Odd-m terms break C(-q) = -conj C(q), so every
- * scan frequency is evaluated. candidates: DEVICE array of n_cand
+ * serves 64, 128, 256, 512 and 1024). Odd-m terms break C(-q) = -conj C(q), so
+ * C is formed at every scan frequency. candidates: DEVICE array of n_cand
  * qssb_full_aberrations_t. Flags: QSSB_FLAG_CHI_FP64 (chi from FP64 q and k,
  * reduced in FP64) and QSSB_FLAG_CHUNKS; the others are ignored. */
 int qssb_loss_batch_full(const float* g_half, const float* bf_geom, const float* q_row,
@@ -582,19 +584,20 @@ int qssb_mse_heads(const float* y, const float* target, int32_t rows, int32_t n_
 int qssb_adam(float* w, float* m, float* v, const float* grad, int64_t n, float lr, float beta1,
               float beta2, float eps, float weight_decay, int32_t step, void* w_bf16,
               void* stream);
+/* qssb_adam for n_tensors (at most 8) parameter tensors in one launch: host
+ * arrays of device pointers, element counts and weight decays; w_bf16[i] may
+ * be NULL. With hyper (device {lr, c1, c2} as
+ * qssb_adam_schedule writes them, or NULL) lr and step are not read. */
+int qssb_adam_multi(int32_t n_tensors, float* const* w, float* const* m, float* const* v,
+                    const float* const* grad, const int64_t* n, const float* weight_decay,
+                    void* const* w_bf16, float lr, float beta1, float beta2, float eps,
+                    int32_t step, const float* hyper, void* stream);
 /* The training schedule on the device, for graph-replayed steps: *step += 1,
  * then hyper[0..2] = {lr0 (1 + cos(pi (step - 1 - first_step) / total_steps))
  * / 2, 1 - beta1^step, 1 - beta2^step} (device float[3], device int32 step;
  * first_step: the step count when this cosine run began). */
 int qssb_adam_schedule(float* hyper, int32_t* step, int32_t first_step, int32_t total_steps,
                        float lr0, float beta1, float beta2, void* stream);
-/* The same for n_tensors (at most 8) parameter tensors in one launch: host
- * arrays of device pointers, element counts and weight decays; w_bf16[i] may
- * be NULL. With hyper (device {lr, c1, c2}, or NULL) lr and step are not read. */
-int qssb_adam_multi(int32_t n_tensors, float* const* w, float* const* m, float* const* v,
-                    const float* const* grad, const int64_t* n, const float* weight_decay,
-                    void* const* w_bf16, float lr, float beta1, float beta2, float eps,
-                    int32_t step, const float* hyper, void* stream);
 /* qssb_adam with the learning rate and bias corrections read from hyper
  * (device {lr, c1, c2}, as qssb_adam_schedule writes them). */
 int qssb_adam_dev(float* w, float* m, float* v, const float* grad, int64_t n, const float* hyper,

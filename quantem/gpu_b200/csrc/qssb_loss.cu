@@ -1031,11 +1031,15 @@ __global__ void __launch_bounds__(256) k_loss_final_sq(const double* __restrict_
 //     of its pixels in registers; at the end of the chunk it adds them to its
 //     own partial planes (column-major), so every element has one writer.
 constexpr int kL256 = 256;
-// Staging of one chunk. Twice the chunk halves the launches and their ramps
-// (16 candidates with C30 at 256^2, their chi as a polynomial: 18.5 ms
-// with 32 MB, 17.0 with 64) and
-// still stays in L2. The quadratic loss at 256^2 keeps 32 MB: the persistent
-// launch holds three such slots in L2 and has the launch sequence's chunks.
+// Staging of one chunk. Twice the chunk halves the launches and their ramps and
+// still stays in L2. ms with 32 and 64 MB: with C30 at 256^2 (1781 BF pixels) 1
+// candidate 1.38 / 1.26, 16 21.1 / 19.2, 64 83.1 / 74.6; at 512^2 (437) 9
+// candidates 9.8 / 8.9, quadratic 8.5 / 7.9; at 1024^2 (109) 1 candidate 1.96 /
+// 1.74, quadratic 1.58 / 1.47; 14 terms at 256^2, 4 candidates 14.7 / 13.6, 512^2,
+// 1 candidate 5.0 / 4.6 (one row a warp). The quadratic loss at 256^2 keeps 32
+// MB, which costs it 7% (16 candidates 19.5 ms, 18.2 with 64): its chunks are
+// those of the persistent launch, which holds three such slots in L2, and so are
+// its bits.
 constexpr size_t kStageBudget = 64u << 20;
 constexpr size_t kStageBudgetQueue = 32u << 20;
 // Set by qssb_loss_batch_ex alone (callers' bit 7 is dropped): a buffer that
@@ -1162,8 +1166,12 @@ static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chu
     return tp;
 }
 
-// One row-pass work item: rows rowblock * RW .. + RW - 1 of BF pixel b0 + bi
-// for candidate cand0 + zc. scr: RW warp FFT scratches; tw: the twiddles
+// One row-pass work item: rows rowblock * row_block .. + row_block - 1 (warp w:
+// every RW-th from w on) of BF pixel b0 + bi for candidate cand0 + zc. The
+// partners C(-r, N/2) of the rows' Nyquist elements are evaluated a lane each by
+// one warp and added by another pass over shared memory; by lane 0 of each row's
+// warp they took 16 candidates with C30 at 256^2 from 19.2 to 20.5 ms, 1 at
+// 512^2 from 1.13 to 1.25. scr: RW warp FFT scratches; tw: the twiddles
 // (filled before the item's first barrier).
 template <int N, bool CHI64, bool QUAD, bool FULL>
 __device__ __forceinline__ void loss_rows_item(
@@ -1750,14 +1758,16 @@ static size_t loss_workspace(const LossPlan& pl) {
 // ticket taken is held by a running CTA, so the batch drains whatever the
 // number of resident CTAs. Producers write through L2 and fence before their
 // counts; consumers read staged rows, deviations and partial planes through
-// L2 only. The chunking is the launch sequence's, and so are the bits on the
-// quadratic path (the general-chi arithmetic, inlined into another kernel,
-// may contract differently: float32 rounding). A wait that runs out, or a set
+// L2 only. On the quadratic path the chunking is the launch sequence's, and so
+// are the bits; batches with C30 have half the sequence's chunk (and the
+// general-chi arithmetic, inlined into another kernel, may contract
+// differently), so they agree to float32 rounding. A wait that runs out, or a set
 // cancel flag, sets the abort word: later items only count themselves and
-// k_loss_final writes NaN losses. CTAs that wait hold their slots; with two
-// staging slots that cost 16% against the launch sequence, with three (96 MB
-// of L2-resident staging at 27 candidates per group) it is 3% faster with C30
-// and 2.5% slower with quadratic chi.
+// k_loss_final writes NaN losses. CTAs that wait hold their slots: with
+// three staging slots (96 MB of L2-resident staging at 27 candidates per group)
+// 64 candidates at 256^2 beside two 128^2 scans' (one graph) take 107.8 ms with
+// C30 against the launch sequence's 97.9, and 95.7 against 89.1 quadratic. It is
+// for callers who want few kernels in a graph (6 and 9 against 947 and 2150).
 struct QueuePlan {
     int K;       // BF chunks over all candidate groups
     int SR, SC;  // items of one row phase, of one column phase
@@ -2151,11 +2161,12 @@ static int dispatch_loss(bool sym, bool chi64, bool quad, const float* g_half, c
 
 // ------------------------------------------------------ 14-term chi
 // Odd-m terms (C21, C23, C41, C43, C45) make chi odd in part, which breaks
-// C(-q) = -conj C(q): every scan frequency is evaluated. N <= 128: the whole
+// C(-q) = -conj C(q), so C is formed at every scan frequency. 128^2 in float32
+// chi: k_loss_full128, chi's even and odd parts shared by q and -q. 64^2, and
+// 128^2 from FP64 chi: k_loss_full, every frequency on its own, the whole
 // N x (N+1) plane in shared memory (k_loss_moments without the mirror).
-// N >= 256: each warp evaluates, inverse-FFTs and stages full rows in the
-// CTA's global plane, then rebuilds its columns from it (k_loss_staged
-// without the row(-r) reconstruction). Partial planes are column-major.
+// N >= 256: the two passes above over all N rows. Partial planes are
+// column-major, k_loss_full128's row-major.
 struct FullConsts {
     Probe p;
     FullChi f;

@@ -14,9 +14,12 @@ library's own count of the kernels captured (``qssb_kernel_launches``).
 The work partition of each scan's loss kernel is chosen by the autotuner
 (``autotune.tune_loss``) before capture. By default (``persistent=True``)
 each 256^2 scan's row and column passes run as one persistent launch
-(``QSSB_FLAG_PERSISTENT``): four kernels for that scan instead of two per BF
-chunk, the same losses to float32 rounding, and faster with C30 candidates;
-``persistent=False`` keeps the launch sequence.
+(``QSSB_FLAG_PERSISTENT``): four kernels for that scan (five for a quadratic
+sweep) instead of two per BF chunk, the same losses to float32 rounding.
+``persistent=False`` keeps the launch sequence, whose graph is larger and
+faster: 64 candidates for each of three scans (96^2, 128^2, 160 x 120) run at
+1962 evaluations/s with C30 (947 kernels) against 1781 (6), and at 2155 (2150
+kernels) against 2007 (9) without.
 """
 from __future__ import annotations
 
