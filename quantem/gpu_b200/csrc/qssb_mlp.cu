@@ -226,14 +226,15 @@ __global__ void __launch_bounds__(256) k_mse_heads(
 // bias corrections come from the device ({lr, c1, c2}, written by
 // k_adam_schedule) instead of the arguments. HBM-bound (30 bytes a parameter
 // with the BF16 copy): a block takes kAdamChunk elements of one tensor, a
-// thread four of them per 16-byte access, and all of its loads are issued
-// before the first update, so that a block keeps 64 KB in flight. The
-// proposer's step (8.9M parameters in 8 tensors): 62 us, against 86 in 8
-// launches of one element per thread and access.
+// thread four of them in one 16-byte access per array. The proposer's step (8.9M
+// parameters in 8 tensors): 42 us, 6.3 TB/s, against 85 in 8 launches of one
+// element per thread and access. Four accesses a thread and array, issued
+// before the first update, took 63 us, and at 2.5M to 4M parameters in one
+// tensor, where their fewer blocks leave a ragged last wave, longer than the one
+// element (2.5M: 14.4 us against 12.4; now 9.8).
 constexpr int kAdamTensors = 8;
 constexpr int kAdamThreads = 256;
-constexpr int kAdamVecs = 4;  // 16-byte accesses per thread and array
-constexpr int kAdamChunk = kAdamThreads * 4 * kAdamVecs;
+constexpr int kAdamChunk = kAdamThreads * 4;
 
 struct AdamTensor {
     float* w;
@@ -274,31 +275,23 @@ __global__ void __launch_bounds__(kAdamThreads) k_adam(const __grid_constant__ A
                      ((((uintptr_t)t.w | (uintptr_t)t.m | (uintptr_t)t.v | (uintptr_t)t.g) & 15u) == 0) &&
                      ((uintptr_t)t.w_bf & 7u) == 0;
     if (vec) {
-        float4 g[kAdamVecs], m[kAdamVecs], v[kAdamVecs], w[kAdamVecs];
-#pragma unroll
-        for (int j = 0; j < kAdamVecs; ++j) {
-            const long long i = base + 4 * (threadIdx.x + j * kAdamThreads);
-            g[j] = __ldcs(reinterpret_cast<const float4*>(t.g + i));
-            m[j] = *reinterpret_cast<const float4*>(t.m + i);
-            v[j] = *reinterpret_cast<const float4*>(t.v + i);
-            w[j] = *reinterpret_cast<const float4*>(t.w + i);
-        }
-#pragma unroll
-        for (int j = 0; j < kAdamVecs; ++j) {
-            const long long i = base + 4 * (threadIdx.x + j * kAdamThreads);
-            update(g[j].x, m[j].x, v[j].x, w[j].x);
-            update(g[j].y, m[j].y, v[j].y, w[j].y);
-            update(g[j].z, m[j].z, v[j].z, w[j].z);
-            update(g[j].w, m[j].w, v[j].w, w[j].w);
-            *reinterpret_cast<float4*>(t.m + i) = m[j];
-            *reinterpret_cast<float4*>(t.v + i) = v[j];
-            *reinterpret_cast<float4*>(t.w + i) = w[j];
-            if (t.w_bf) {
-                const __nv_bfloat162 lo = __floats2bfloat162_rn(w[j].x, w[j].y);
-                const __nv_bfloat162 hi = __floats2bfloat162_rn(w[j].z, w[j].w);
-                *reinterpret_cast<uint2*>(t.w_bf + i) = make_uint2(
-                    *reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-            }
+        const long long i = base + 4 * threadIdx.x;
+        const float4 g = __ldcs(reinterpret_cast<const float4*>(t.g + i));
+        float4 m = *reinterpret_cast<const float4*>(t.m + i);
+        float4 v = *reinterpret_cast<const float4*>(t.v + i);
+        float4 w = *reinterpret_cast<const float4*>(t.w + i);
+        update(g.x, m.x, v.x, w.x);
+        update(g.y, m.y, v.y, w.y);
+        update(g.z, m.z, v.z, w.z);
+        update(g.w, m.w, v.w, w.w);
+        *reinterpret_cast<float4*>(t.m + i) = m;
+        *reinterpret_cast<float4*>(t.v + i) = v;
+        *reinterpret_cast<float4*>(t.w + i) = w;
+        if (t.w_bf) {
+            const __nv_bfloat162 lo = __floats2bfloat162_rn(w.x, w.y);
+            const __nv_bfloat162 hi = __floats2bfloat162_rn(w.z, w.w);
+            *reinterpret_cast<uint2*>(t.w_bf + i) = make_uint2(
+                *reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
         }
         return;
     }

@@ -283,18 +283,18 @@ def test_forward_model_features_match_simulated_scans():
 
 
 def test_adam_multi_takes_remainders_and_unaligned_tensors():
-    """One launch over tensors around the 4096-element block and off 16-byte
+    """One launch over tensors around the 1024-element block and off 16-byte
     alignment, with and without the BF16 copy; a dozen float32 operations per
     element, each within 2^-24: 2e-6 of the update's scale."""
-    sizes = [1, 4095, 4096, 4097, 9000]
+    sizes = [1, 1023, 1024, 1025, 4095, 4096, 4097, 9000]
     g = torch.Generator(device=DEV).manual_seed(3)
     rnd = lambda n, off: torch.randn(n + off, device=DEV, generator=g)[off:]  # noqa: E731
-    offs = [0, 0, 0, 0, 1]
+    offs = [0, 0, 0, 0, 1, 0, 0, 1]
     w, m, grad = ([rnd(n, o) for n, o in zip(sizes, offs)] for _ in range(3))
     v = [rnd(n, o).square() for n, o in zip(sizes, offs)]
     copy = [torch.empty(n, dtype=torch.bfloat16, device=DEV) if i % 2 else None
             for i, n in enumerate(sizes)]
-    wd = [0.1, 0.0, 0.2, 0.0, 0.3]
+    wd = [0.1, 0.0, 0.2, 0.0, 0.3, 0.0, 0.1, 0.2]
     lr, b1, b2, eps, step, k = 1e-2, 0.9, 0.999, 1e-8, 3, len(sizes)
     want = []
     for i in range(k):
