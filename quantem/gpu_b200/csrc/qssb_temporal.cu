@@ -212,22 +212,27 @@ __device__ __forceinline__ double2 warp_sum(double2 v) {
     return v;
 }
 
-// partial[t][blk] = sum over this block's pixels of a_t conj(a_0), FP64.
+// partial[t][blk] = sum over this block's pixels of a_t conj(a_0), FP64. FULL:
+// kJoinBlocks blocks a frame, a stride that the compiler knows, two pixels'
+// loads at once (64 frames of 1024^2: 97 us; 137 with four, 118 with a stride of
+// gridDim.x).
+template <bool FULL>
 __global__ void __launch_bounds__(kJoinThreads) k_overlap_partial(const float2* __restrict__ a,
                                                                   long long n_pix,
                                                                   double2* __restrict__ partial) {
     __shared__ double2 red[kJoinThreads / 32];
     const int t = blockIdx.y;
     const float2* at = a + (size_t)t * n_pix;
-    double2 sum = make_double2(0.0, 0.0);
-    for (long long p = (long long)blockIdx.x * kJoinThreads + threadIdx.x; p < n_pix;
-         p += (long long)gridDim.x * kJoinThreads) {
+    double sr = 0.0, si = 0.0;
+    const long long stride = (long long)(FULL ? kJoinBlocks : gridDim.x) * kJoinThreads;
+#pragma unroll(FULL ? 2 : 1)
+    for (long long p = (long long)blockIdx.x * kJoinThreads + threadIdx.x; p < n_pix; p += stride) {
         const float2 v = at[p];
         const float2 r = a[p];
-        sum.x += (double)v.x * r.x + (double)v.y * r.y;
-        sum.y += (double)v.y * r.x - (double)v.x * r.y;
+        sr += (double)v.x * r.x + (double)v.y * r.y;
+        si += (double)v.y * r.x - (double)v.x * r.y;
     }
-    sum = warp_sum(sum);
+    double2 sum = warp_sum(make_double2(sr, si));
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -246,6 +251,10 @@ __global__ void __launch_bounds__(128) k_overlap_rotation(const double2* __restr
     const int t = blockIdx.x * 4 + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (t >= n_frames) return;
+    if (t == 0) {
+        if (lane == 0) rot[0] = make_float2(1.0f, 0.0f);
+        return;
+    }
     double2 sum = make_double2(0.0, 0.0);
     for (int b = lane; b < n_blocks; b += 32) {
         const double2 v = partial[(size_t)t * n_blocks + b];
@@ -255,13 +264,13 @@ __global__ void __launch_bounds__(128) k_overlap_rotation(const double2* __restr
     sum = warp_sum(sum);
     if (lane != 0) return;
     const double ang = atan2(sum.y, sum.x);
-    rot[t] = t == 0 ? make_float2(1.0f, 0.0f) : make_float2((float)cos(ang), (float)-sin(ang));
+    rot[t] = make_float2((float)cos(ang), (float)-sin(ang));
 }
 
 // joined[p] = sum_t w_t rot_t a_t[p] in FP32; the rotated frames are written
 // back when requested. A block takes 32 pixels and its 8 warps every 8th
 // frame, the 8 sums added in order: a thread per pixel over all frames leaves
-// 64 blocks at 128^2 (52 us for 256 frames).
+// 64 blocks at 128^2.
 constexpr int kJoinSlices = kJoinThreads / 32;
 __global__ void __launch_bounds__(kJoinThreads) k_join(float2* __restrict__ a,
                                                        const float* __restrict__ w,
@@ -295,6 +304,34 @@ __global__ void __launch_bounds__(kJoinThreads) k_join(float2* __restrict__ a,
     }
     joined[p] = make_float2(sr, si);
 }
+
+// The same by a thread per pixel, all frames in order.
+__global__ void __launch_bounds__(kJoinThreads) k_join_pixels(float2* __restrict__ a,
+                                                              const float* __restrict__ w,
+                                                              const float2* __restrict__ rot,
+                                                              int n_frames, long long n_pix,
+                                                              float2* __restrict__ joined,
+                                                              int write_back) {
+    const long long p = (long long)blockIdx.x * kJoinThreads + threadIdx.x;
+    if (p >= n_pix) return;
+    float sr = 0.0f, si = 0.0f;
+#pragma unroll 4
+    for (int t = 0; t < n_frames; ++t) {
+        float2 v = a[(size_t)t * n_pix + p];
+        if (rot) v = cmul(v, __ldg(rot + t));
+        if (write_back) a[(size_t)t * n_pix + p] = v;
+        const float wt = __ldg(w + t);
+        sr = fmaf(wt, v.x, sr);
+        si = fmaf(wt, v.y, si);
+    }
+    joined[p] = make_float2(sr, si);
+}
+
+// Pixels from which a thread each fills the chip. k_join against k_join_pixels,
+// us: 256 frames of 128^2 9 / 47, 64 of 256^2 9.0 / 14.4, 256 of 256 x 512 70 /
+// 121; 16 of 512^2 10.3 / 8.9 and 64 of them 37 / 36, 1 of 1024^2 20 / 9, 16 of
+// them 51 / 37.
+constexpr long long kJoinPixels = 1 << 18;
 
 template <int C>
 static int launch_rows(const float2* in, float2* out, int n_frames, int rows, const float* shifts,
@@ -385,15 +422,30 @@ extern "C" int qssb_join_object_waves(float* frames, const float* weights, int32
         const size_t part = (sizeof(double2) * (size_t)n_frames * kJoinBlocks + 255) & ~(size_t)255;
         rot = reinterpret_cast<float2*>(static_cast<char*>(workspace) + part);
         const int n_blocks = overlap_blocks(n_pix);
-        { k_overlap_partial<<<dim3(n_blocks, n_frames), kJoinThreads, 0, s>>>(a, n_pix, partial); note_launch(); }
+        auto launch_partial = [&](auto kern) {
+            kern<<<dim3(n_blocks, n_frames), kJoinThreads, 0, s>>>(a, n_pix, partial);
+            note_launch();
+        };
+        if (n_blocks == kJoinBlocks)
+            launch_partial(k_overlap_partial<true>);
+        else
+            launch_partial(k_overlap_partial<false>);
         CUDA_TRY(cudaGetLastError());
         { k_overlap_rotation<<<(n_frames + 3) / 4, 128, 0, s>>>(partial, n_blocks, n_frames, rot); note_launch(); }
         CUDA_TRY(cudaGetLastError());
     }
-    const long long blocks = (n_pix + 31) / 32;
+    const int per_block = n_pix < kJoinPixels ? 32 : kJoinThreads;
+    const long long blocks = (n_pix + per_block - 1) / per_block;
     if (blocks > 0x7fffffffLL) return set_error(QSSB_ERR_INVALID, "qssb_join_object_waves: too many pixels");
-    { k_join<<<(unsigned)blocks, kJoinThreads, 0, s>>>(a, weights, rot, n_frames, n_pix,
-                                                     reinterpret_cast<float2*>(joined), write_back); note_launch(); }
+    auto launch = [&](auto kern) {
+        kern<<<(unsigned)blocks, kJoinThreads, 0, s>>>(a, weights, rot, n_frames, n_pix,
+                                                       reinterpret_cast<float2*>(joined), write_back);
+        note_launch();
+    };
+    if (n_pix < kJoinPixels)
+        launch(k_join);
+    else
+        launch(k_join_pixels);
     CUDA_TRY(cudaGetLastError());
     return QSSB_OK;
 }

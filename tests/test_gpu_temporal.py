@@ -145,11 +145,12 @@ def test_time_series_through_ssb_sessions():
         s.close()
 
 
-@pytest.mark.parametrize("shape", [(64, 128), (128, 64), (128, 1024)])
+@pytest.mark.parametrize("shape", [(64, 128), (128, 64), (128, 1024), (512, 512)])
 @pytest.mark.parametrize("n", [1, 8, 9, 67])
 def test_join_slices_and_strips(shape, n):
     """Frame counts around the join's 8 slices, columns and rows fewer than,
-    equal to and more than a block's 32 lines; float32 sums, 3e-6 as above."""
+    equal to and more than a block's 32 lines, and the first size whose join
+    takes a thread per pixel; float32 sums, 3e-6 as above."""
     rng = np.random.default_rng(n + shape[0])
     waves = rng.standard_normal((n, *shape)) + 1j * rng.standard_normal((n, *shape))
     shifts = rng.uniform(-6.0, 6.0, (n, 2))
