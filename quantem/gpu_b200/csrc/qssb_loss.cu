@@ -1068,15 +1068,18 @@ static bool loss_queue_requested(int n, int flags) {
 // CTAs per SM (80 registers) hide more latency than one 16-warp CTA at 128.
 __host__ __device__ constexpr int row_warps(int n) { return n >= 1024 ? 8 : (n == 256 ? 8 : 16); }
 __host__ __device__ constexpr int row_min_ctas(int n) { return n == 256 ? 3 : 1; }
-// The 14-term chi's CTA starts with FP64 work (its coefficients, P(k)), shared
-// by four rows a warp up to 512^2. One row a warp against four, with the plan's
-// chunk that fills the waves: 2 candidates of 1781 BF pixels at 256^2 8.6 / 6.8
-// ms, of 437 at 512^2 9.2 / 7.4 (9 candidates 40.1 / 31.9); at 1024^2, where a
-// row is 32 values a lane, 1 candidate of 109 BF pixels 7.3 / 7.5, 4 candidates
-// 29.9 / 28.9. The half set has no such start: with four rows at 256^2 a batch
-// with C30 takes 8% longer (16 candidates: 19.2 / 20.8 ms), a quadratic one 12%
-// (19.5 / 21.7) and from a full group of 27 on 6% less (30.3 / 28.4).
-__host__ __device__ constexpr int rows_per_warp(int n, bool full) { return full && n <= 512 ? 4 : 1; }
+// Rows per warp of the 14-term chi's row pass. Its CTA starts with FP64 work
+// (its coefficients, P(k)), which four rows a warp share up to 512^2 where the
+// chunk's CTAs of four fill three quarters of their slots; fewer leave SMs idle.
+// One row against four, 1 candidate: 256^2 and 13 BF pixels (104 CTAs of 444
+// slots) 92 / 142 us, 45 (360) 176 / 167, 421 1138 / 919; 512^2 and 13 (104 of
+// 148) 190 / 228, 421 4.34 / 3.65 ms. At 1024^2, where a row is 32 values a lane,
+// 109 BF pixels 7.3 / 7.5 ms and 4 candidates 29.9 / 28.9: one row. The half set
+// has no such start: with four rows at 256^2 a batch with C30 takes 8% longer (16
+// candidates of 1781 BF pixels: 19.2 / 20.8 ms), a quadratic one 12% (19.5 / 21.7)
+// and from a full group of 27 on 6% less (30.3 / 28.4).
+constexpr int kFullRows = 4;
+__host__ __device__ constexpr bool shared_rows(int n, bool full) { return full && n <= 512; }
 __host__ __device__ constexpr int row_load_batch(int n) { return n == 256 ? 4 : 8; }
 __host__ __device__ constexpr int col_tile(int n) { return n >= 1024 ? 8 : 16; }
 
@@ -1088,9 +1091,7 @@ struct TwoPass {
     // CTA after its row 0, so the rows 0 .. N/2 - 1 fill whole CTAs (17 CTAs
     // of 8 warps would leave one CTA a single row)
     static constexpr bool fold_nyquist = !FULL && N == 256;
-    static constexpr int row_block = rwarps * rows_per_warp(N, FULL);  // rows of one CTA
-    static constexpr int row_ctas =
-        fold_nyquist ? N / 2 / row_block : (rows + row_block - 1) / row_block;
+    static constexpr int row_ctas = fold_nyquist ? N / 2 / rwarps : (rows + rwarps - 1) / rwarps;
     static constexpr int tile = col_tile(N);
     static constexpr int scratch = warp_fft_scratch<N>();
     // column line pitch: odd mod 16 (conflict-free strip loads), and room for
@@ -1138,13 +1139,12 @@ static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chu
     const size_t per_bf = sizeof(float2) * (size_t)(full ? n : n / 2 + 1) * n;
     long long c = (long long)(budget / (per_bf * (size_t)group));
     if (c < 1) c = 1;
-    if (rows_per_warp(n, full) > 1) {
+    if (shared_rows(n, full)) {
         // the chunk, from the budget down to half of it, whose row pass fills its
-        // waves best (an item is 32 or 64 rows, so a last wave is a larger share:
-        // 2 candidates at 256^2 7.4 ms with the budget's chunk, 6.8 with this one,
-        // 9 at 512^2 40.5 and 31.9)
-        const int ctas = n == 256 ? TwoPass<256, true>::row_ctas : TwoPass<512, true>::row_ctas;
-        const long long items = (long long)ctas * group;
+        // waves best (an item is 32 or 64 rows, so a last wave is a larger share: 2
+        // candidates of 1781 BF pixels at 256^2 7.4 ms with the budget's chunk, 6.8
+        // with this one, 9 of 437 at 512^2 40.5 and 31.9)
+        const long long items = (long long)(n / (row_warps(n) * kFullRows)) * group;
         const long long rslots = 148LL * row_min_ctas(n);
         double best = 0.0;
         for (long long k = c, kmin = (c + 1) / 2; k >= kmin; --k) {
@@ -1166,8 +1166,9 @@ static TwoPassPlan plan_two_pass(int n, bool full, int n_bf, int n_cand, int chu
     return tp;
 }
 
-// One row-pass work item: rows rowblock * row_block .. + row_block - 1 (warp w:
-// every RW-th from w on) of BF pixel b0 + bi for candidate cand0 + zc. The
+// One row-pass work item: RW * n_rows rows from rowblock on (warp w: every RW-th
+// of them; n_rows is 1 for the half set) of BF pixel b0 + bi for candidate
+// cand0 + zc. The
 // partners C(-r, N/2) of the rows' Nyquist elements are evaluated a lane each by
 // one warp and added by another pass over shared memory; by lane 0 of each row's
 // warp they took 16 candidates with C30 at 256^2 from 19.2 to 20.5 ms, 1 at
@@ -1180,7 +1181,7 @@ __device__ __forceinline__ void loss_rows_item(
     const qssb_calibration_t& cal, const Probe* __restrict__ probes,
     const float2* __restrict__ eq_table, int cand0, int b0, int nb_chunk,
     float2* __restrict__ stage, float2* __restrict__ delta, const float2* __restrict__ overlap,
-    int rowblock, int bi, int zc, float2* scr, const float2* tw) {
+    int rowblock, int n_rows, int bi, int zc, float2* scr, const float2* tw) {
     using TP = TwoPass<N, FULL>;
     constexpr int H = N / 2 + 1;
     constexpr int RW = TP::rwarps;
@@ -1190,18 +1191,17 @@ __device__ __forceinline__ void loss_rows_item(
     __shared__ FullChi sf;
     __shared__ FullChi64 sd;
     __shared__ float2 s_phc[kSep ? N : 1];
-    constexpr int RB = TP::row_block;
-    __shared__ float2 s_phr[kSep ? RB : 1];
+    __shared__ float2 s_phr[kSep ? RW : 1];
     // the Nyquist column of the CTA's rows: conj C(r, N/2) and C(-r, N/2)
-    __shared__ float2 s_ny[FULL ? 1 : RB];
-    __shared__ float2 s_partner[FULL ? 1 : RB];
-    static_assert(FULL || RB <= 32, "one warp evaluates the partners");
+    __shared__ float2 s_ny[FULL ? 1 : RW];
+    __shared__ float2 s_partner[FULL ? 1 : RW];
+    static_assert(FULL || RW <= 32, "one warp evaluates the partners");
     const int tid = threadIdx.x;
     const int lane = tid & 31;
     const int warp = tid >> 5;
     const int b = b0 + bi;
     const int cand = cand0 + zc;
-    const int r0 = rowblock * RB;
+    const int r0 = rowblock * RW * (FULL ? n_rows : 1);
     {  // the candidate's probe, from k_two_pass_setup
         const auto* src = reinterpret_cast<const unsigned int*>(probes + cand);
         auto* dst = reinterpret_cast<unsigned int*>(&sp);
@@ -1225,7 +1225,7 @@ __device__ __forceinline__ void loss_rows_item(
                                 __ldg(geom + 4 * n_bf + b), __ldg(geom + 5 * n_bf + b), p);
     }
     if constexpr (kSep) {  // e^{i 2 q_col(c) v} for all columns, e^{i 2 q_row(r) u} for this CTA's rows
-        for (int i = tid; i < N + RB; i += 32 * RW) {
+        for (int i = tid; i < N + RW; i += 32 * RW) {
             float sn, cs;
             if (i < N) {
                 sincosf(2.0f * __ldg(q_col + i) * kq.v, &sn, &cs);
@@ -1307,7 +1307,7 @@ __device__ __forceinline__ void loss_rows_item(
     if constexpr (!FULL) {
         // the partners C(-r, N/2) of the CTA's rows, one lane each
         const int r = r0 + lane;
-        if (warp == RW - 1 && lane < RB && r >= 1 && r < N / 2) {
+        if (warp == RW - 1 && lane < RW && r >= 1 && r < N / 2) {
             float2 e_neg = make_float2(1.0f, 0.0f);
             if constexpr (kSep) {
                 float sn, cs;
@@ -1322,7 +1322,7 @@ __device__ __forceinline__ void loss_rows_item(
         }
     }
 #pragma unroll 1
-    for (int j = 0; j < rows_per_warp(N, FULL); ++j) {
+    for (int j = 0; j < (FULL ? n_rows : 1); ++j) {
         const int r = r0 + warp + RW * j;
         if (r >= TP::rows) break;
         row(r, kSep ? s_phr[r - r0] : make_float2(1.0f, 0.0f));
@@ -1331,11 +1331,11 @@ __device__ __forceinline__ void loss_rows_item(
     if constexpr (!FULL) {
         __syncthreads();
         const int r = r0 + tid;
-        if (tid < RB && r >= 1 && r < N / 2)
+        if (tid < RW && r >= 1 && r < N / 2)
             delta[((size_t)zc * nb_chunk + bi) * (N / 2) + r] = cadd(s_ny[tid], s_partner[tid]);
     }
     if constexpr (TP::fold_nyquist) {
-        static_assert(TP::row_ctas * RB == N / 2, "whole CTAs of rows");
+        static_assert(TP::row_ctas * RW == N / 2, "whole CTAs of rows");
         if (rowblock == 0 && warp == 0) {
             float2 e_row = make_float2(1.0f, 0.0f);
             if constexpr (kSep) {
@@ -1353,7 +1353,7 @@ __global__ void __launch_bounds__(32 * row_warps(N), row_min_ctas(N)) k_loss_row
     const float2* __restrict__ g, int n_bf, const float* __restrict__ geom,
     const float* __restrict__ q_row, const float* __restrict__ q_col, const void* __restrict__ cands,
     qssb_calibration_t cal, const Probe* __restrict__ probes, const float2* __restrict__ twg,
-    const float2* __restrict__ eq_table, int cand0, int b0, int nb_chunk,
+    const float2* __restrict__ eq_table, int cand0, int b0, int nb_chunk, int n_rows,
     float2* __restrict__ stage, float2* __restrict__ delta, const float2* __restrict__ overlap) {
     using TP = TwoPass<N, FULL>;
     extern __shared__ float4 smem4[];
@@ -1362,7 +1362,7 @@ __global__ void __launch_bounds__(32 * row_warps(N), row_min_ctas(N)) k_loss_row
     for (int i = threadIdx.x; i < N; i += 32 * TP::rwarps) tw[i] = __ldg(twg + i);
     loss_rows_item<N, CHI64, QUAD, FULL>(g, n_bf, geom, q_row, q_col, cands, cal, probes,
                                          eq_table, cand0, b0, nb_chunk, stage, delta, overlap,
-                                         blockIdx.x, blockIdx.y, blockIdx.z, scr, tw);
+                                         blockIdx.x, n_rows, blockIdx.y, blockIdx.z, scr, tw);
 }
 
 __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gmem_src) {
@@ -1890,7 +1890,7 @@ __global__ void __launch_bounds__(32 * TwoPass<N, false>::rwarps, 3) k_loss_queu
                 if (zc < qp.nc[gi] && bi < nb)
                     loss_rows_item<N, false, QUAD, false>(g, n_bf, geom, q_row, q_col, cands, cal,
                                                           probes, eq_table, qp.c0[gi], b0, nb, st,
-                                                          dl, overlap, rb, bi, zc, scr, tw);
+                                                          dl, overlap, rb, 1, bi, zc, scr, tw);
             } else {
                 const int strip = w % kStrips;
                 const int rest = w / kStrips;
@@ -2030,10 +2030,16 @@ static int launch_two_pass(const float* g_half, const float* geom, const float* 
         if (chunk > cal.n_bf) chunk = cal.n_bf;
         for (int b0 = 0; b0 < cal.n_bf; b0 += chunk) {
             const int nb = cal.n_bf - b0 < chunk ? cal.n_bf - b0 : chunk;
+            int n_rows = 1, row_ctas = TP::row_ctas;
+            if (shared_rows(N, FULL) &&
+                4LL * (TP::row_ctas / kFullRows) * nb * nc >= 3LL * 148 * row_min_ctas(N)) {
+                n_rows = kFullRows;
+                row_ctas = TP::row_ctas / kFullRows;
+            }
             { k_loss_rows<N, CHI64, QUAD, FULL>
-                <<<dim3(TP::row_ctas, nb, nc), 32 * TP::rwarps, TP::row_smem, s>>>(
+                <<<dim3(row_ctas, nb, nc), 32 * TP::rwarps, TP::row_smem, s>>>(
                     g, cal.n_bf, geom, q_row, q_col, cands, cal, probes, twg, eq, c0, b0, nb,
-                    stage, delta, overlap); note_launch(); }
+                    n_rows, stage, delta, overlap); note_launch(); }
             CUDA_TRY(cudaGetLastError());
             if constexpr (TP::pair_cols) {
                 { k_loss_cols_pair<N><<<dim3(N / TP::tile, pl.n_chunks, nc), 32 * TP::pair_warps,

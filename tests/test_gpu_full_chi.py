@@ -167,11 +167,13 @@ def test_paired_evaluation_matches_the_fp64_chi_kernel(chunks, det_sampling):
     be.close()
 
 
-def test_512_rows_in_groups_match_the_symmetric_path():
-    """k_loss_rows<512, FULL> (four rows a warp, chunks that fill its waves)
-    with C10, C12 and C30 only, against the half-set kernels, for a group of
-    candidates and one beyond it; 27 BF pixels, float32 sums: 2e-6."""
-    counts = disk_input(123, scan=(512, 512))
+@pytest.mark.parametrize("scan", [256, 512])
+def test_row_blocks_and_groups_match_the_symmetric_path(scan):
+    """k_loss_rows<FULL> with C10, C12 and C30 only against the half-set
+    kernels, 27 BF pixels: one candidate (too few CTAs for four rows a warp at
+    256^2, a chunk of four rows and one of one row at 512^2) and ten (four rows;
+    more than a group at 512^2). Float32 sums: 2e-6."""
+    counts = disk_input(123, scan=(scan, scan))
     be = B200SSBBackend(torch.as_tensor(counts, device=DEV), semiangle=21.4, scan_sampling=0.5,
                         det_sampling=1.0, voltage_kV=300, bf_radius=3)
     for n in (1, 10):
