@@ -943,8 +943,11 @@ __device__ __forceinline__ void corrected_full_pair(float qx, float qy, float qx
         am = soft_aperture_fp64(qx64 - kx64, qy64 - ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
         ap = soft_aperture_fp64(qx64 + kx64, qy64 + ky64, p.semi_d, p.lam_d, p.ang_r_d, p.ang_c_d);
     }
-    v = v_neg = make_float2(0.0f, 0.0f);
-    if (am == 0.0f && ap == 0.0f) return;  // Gamma == 0
+    if (am == 0.0f && ap == 0.0f) {  // Gamma == 0: nothing of a finite G, NaN of any other
+        v = make_float2(0.0f * g.x, 0.0f * g.y);
+        v_neg = cconj(v);
+        return;
+    }
     const float2 xc = __fadd2_rn(x, make_float2(qx_lo - kx_lo, qx_lo + kx_lo));
     const float2 yc = __fadd2_rn(y, make_float2(qy_lo - ky_lo, qy_lo + ky_lo));
     float2 even, odd;

@@ -185,3 +185,15 @@ def test_row_blocks_and_groups_match_the_symmetric_path(scan):
         want = be.variance_loss_batch(mags[:, 0], mags[:, 1], angs[:, 1], mags[:, 4])
         torch.testing.assert_close(got, want, rtol=2e-6, atol=0)
     be.close()
+
+
+@pytest.mark.parametrize("value", [math.nan, math.inf])
+@pytest.mark.parametrize("chi_fp64", [False, True])
+def test_a_spectrum_that_is_not_finite_gives_a_nan_loss(value, chi_fp64):
+    """One element of G beyond every aperture: not a loss of the others."""
+    be, _ = _case(128, chi_fp64)
+    mags, angs = np.array(MAGS), np.array(ANGS)
+    assert np.isfinite(float(be.variance_loss_batch_full(mags, angs)[0]))
+    be.G_qk[3, 60, 62] = complex(value, 0.0)
+    assert np.isnan(float(be.variance_loss_batch_full(mags, angs)[0]))
+    be.close()
